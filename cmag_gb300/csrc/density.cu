@@ -75,15 +75,14 @@ __device__ __forceinline__ void wendland_run(const DevParams &p, const float4 *_
         float2 t = __ffma2_rn(d, nh2, one);   // 1 - q/2
         t = make_float2(fmaxf(t.x, 0.0f), fmaxf(t.y, 0.0f));  // 0 outside the support (q >= 2)
         const float2 t2 = __fmul2_rn(t, t);
-        const float2 w = __fmul2_rn(__fmul2_rn(t2, t2), __ffma2_rn(d, h2, one));  // ... (2q + 1)
-        acc = __fadd2_rn(acc, w);
+        acc = __ffma2_rn(__fmul2_rn(t2, t2), __ffma2_rn(d, h2, one), acc);  // ... (2q + 1)
         if (LIST && record) {
             const uint32_t v = j | code;  // j + 1 < 2^26: the next entry is v + 1
             if (records<SYS, TRIM, LIST == kKeptList>(p, i, j, d2.x, a.w)) list_append(nl, i, cnt, v);
             if (records<SYS, TRIM, LIST == kKeptList>(p, i, j + 1, d2.y, c.w)) list_append(nl, i, cnt, v + 1u);
         }
     }
-    if (j < e) {  // the same operations as one half of a pair step
+    if (j < e) {  // one half of a pair step, its weight rounded before the sum
         const float4 pj = __ldg(spos + j);
         const float3 r = rel<SYS>(pi, pj, sx, sy, sz);
         const float dxy = __fmaf_rn(r.y, r.y, __fmul_rn(r.x, r.x));
@@ -307,8 +306,7 @@ __global__ void __launch_bounds__(256, 8)
                 float2 t = __ffma2_rn(d, nh2, one);
                 t = make_float2(fmaxf(t.x, 0.0f), fmaxf(t.y, 0.0f));
                 const float2 t2 = __fmul2_rn(t, t);
-                const float2 w = __fmul2_rn(__fmul2_rn(t2, t2), __ffma2_rn(d, h2, one));
-                acc = __fadd2_rn(acc, w);
+                acc = __ffma2_rn(__fmul2_rn(t2, t2), __ffma2_rn(d, h2, one), acc);
             }
             if (k < cnt) {
                 const uint32_t en = __ldg(ep + (size_t)k * nl.stride);

@@ -9,37 +9,16 @@
 #include <cuda_runtime.h>
 
 #include "kernels.h"
+#include "particle_motion.cuh"
 
 namespace cmag {
 
 namespace {
 
-// Advance one boundary-configuration phase exactly as the host mirror does
-// (separately rounded adds and multiplies, no contraction).
-__device__ __forceinline__ void advance_phase(const DevParams &p, PhaseState *ph, float k_milli)
-{
-    PhaseState s = *ph;
-    s.configure = 0;
-    if (s.is_bc) {
-        s.time_shift = __fadd_rn(s.time_shift, p.dt);
-        if (s.wave_height < p.amplitude) {
-            s.configure = 1;
-            s.configure_height = s.wave_height;
-            s.wave_height = __fadd_rn(s.wave_height, __fmul_rn(p.dt, k_milli));
-        } else {
-            s.time_relax = __fsub_rn(s.time_relax, p.dt);
-            if (s.time_relax < 0.0f) s.is_bc = 0;
-        }
-    }
-    s.t = s.is_bc ? 0.0f : __fsub_rn(s.elapsed, s.time_shift);
-    s.elapsed = __fadd_rn(s.elapsed, p.dt);
-    *ph = s;
-}
-
 __global__ void k_phase(DevParams p, PhaseState *ph, float k_milli)
 {
     pdl_entry();
-    advance_phase(p, ph, k_milli);
+    *ph = next_phase(p, *ph, k_milli);
 }
 
 __global__ void k_phase_batch(const DevParams *__restrict__ scenes, uint32_t nscenes,
@@ -47,7 +26,7 @@ __global__ void k_phase_batch(const DevParams *__restrict__ scenes, uint32_t nsc
 {
     pdl_entry();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < nscenes && scenes[s].system == CMAG_PERISTALSIS) advance_phase(scenes[s], ph + s, k_milli);
+    if (s < nscenes && scenes[s].system == CMAG_PERISTALSIS) ph[s] = next_phase(scenes[s], ph[s], k_milli);
 }
 
 // Kept neighbour lists: flag the next step's rebuild when the particle is now
@@ -104,12 +83,8 @@ __global__ void __launch_bounds__(256)
         float4 a = acc[i];
         ax = a.x; ay = a.y; az = a.z;
     } else {
-        const int is_bc = ph->is_bc;
-        if (q.w != 0.0f && is_bc) return;  // walls frozen while configuring
-        if (q.w != 0.0f) {                 // moving walls
-            const float wave = get_wave(p, q.x, ph->t);
-            if (q.w > 0.0f) q.y = -p.half_fluid_h + p.amplitude * wave - p.r * (q.w - 1.0f);
-            else q.y = p.half_fluid_h - p.amplitude * wave + p.r * (-q.w - 1.0f);
+        if (q.w != 0.0f) {
+            if (!move_wall(p, ph->is_bc, ph->t, q)) return;
             pos[i] = q;
             if (xb) check_moved(p, q, xb[i], moved);
             return;
@@ -117,26 +92,9 @@ __global__ void __launch_bounds__(256)
         float4 fv = vforce[i], fp = pforce[i];
         ax = fv.x + fp.x; ay = fv.y + fp.y; az = fv.z + fp.z;
     }
-    float4 v = vel[i];
-    const float nvx = v.x + (p.gvx + ax) * p.dt;
-    const float nvy = v.y + (p.gvy + ay) * p.dt;
-    const float nvz = v.z + (p.gvz + az) * p.dt;
-    const float4 lf = vlf[i];
-    vlf[i] = make_float4((v.x + nvx) * 0.5f, (v.y + nvy) * 0.5f, (v.z + nvz) * 0.5f, lf.w);
-    v.x = nvx; v.y = nvy; v.z = nvz;
-    q.x += v.x * p.dt; q.y += v.y * p.dt; q.z += v.z * p.dt;
-    if (p.system == CMAG_DAMBREAK) {
-        if (q.x < p.left_border) { q.x = p.left_border; v.x *= p.damping; }
-        if (q.x > p.right_boundary) { q.x = p.right_boundary; v.x *= p.damping; }
-        if (q.y < p.bottom_border) { q.y = p.bottom_border; v.y *= p.damping; }
-        if (p.clamp_z) {
-            if (q.z < p.z_min_border) { q.z = p.z_min_border; v.z *= p.damping; }
-            if (q.z > p.z_max_border) { q.z = p.z_max_border; v.z *= p.damping; }
-        }
-    } else {
-        if (q.x > p.half_world_x) q.x -= 2.0f * p.half_world_x;
-        if (p.system == CMAG_PERISTALSIS && q.x < -p.half_world_x) q.x += 2.0f * p.half_world_x;
-    }
+    float4 v = vel[i], lf = vlf[i];
+    integrate_fluid(p, ax, ay, az, q, v, lf);
+    vlf[i] = lf;
     pos[i] = q;
     vel[i] = v;
     if (xb) check_moved(p, q, xb[i], moved);

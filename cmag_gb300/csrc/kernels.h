@@ -168,6 +168,28 @@ void launch_verlet_decide(VerletFlags *flags, unsigned long long cond, int use_c
 void launch_verlet_check(const float4 *pos, const float4 *xb, uint32_t start, uint32_t count, float move2,
                          uint32_t *moved, cudaStream_t st);
 
+// ---- the step of a small planar scene in three launches (small_step.cu) ----------
+// Largest scene that takes it.  The neighbour loops' 8 lanes cost several times the
+// instructions of one lane, which pays while the GPU has idle issue slots: three
+// solvers in turn, us per step of each, here / staged: 352 particles 6.2 / 15.7,
+// 3,840 11 / 21, 16,384 20.5 / 23.8, 21,200 22.3 / 19.8, 34,800 33 / 21.
+constexpr uint32_t kSmallParticles = 18000;
+constexpr uint32_t kSmallCells = 1u << 18;  // the sort's cluster scans them in a few us
+// The arrays of launch_hash .. launch_integrate; rank may alias idx.
+struct SmallStep {
+    float4 *pos, *vel, *vlf, *meas, *spos, *svel;
+    float4 *out_a, *out_b;  // acceleration; or viscous and pressure force
+    float2 *aux;
+    uint32_t *hash, *rank, *shash, *tmp, *idx, *cnt, *off, *err;
+    PhaseState *phase;
+    float k_milli;
+};
+// Whether the scene is of this kind (single planar scenes, one lane per particle).
+bool small_step_fits(const DevParams &p);
+// Blocks of the cluster the current device can run for it (0: none).
+uint32_t small_step_cluster(const DevParams &p);
+cudaError_t launch_small_step(const DevParams &p, const SmallStep &a, uint32_t cluster, cudaStream_t st);
+
 // ---- reductions over fluid particles (reduce.cu) -------------------------------
 // out6: order-preserving keys of min x,y,z then max x,y,z (init 0xffffffff, 0)
 void launch_fluid_extent(int32_t system, const float4 *pos, uint32_t n, uint32_t *out6,

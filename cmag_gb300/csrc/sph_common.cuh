@@ -193,13 +193,13 @@ __device__ __forceinline__ uint32_t grid_hash(const DevParams &p, int gx, int gy
 // 4x4x4 cell block with this step's stamp; a non-fluid particle whose position
 // or type differs from its snapshot takes the new one and marks the cached
 // densities stale (the next scan kernel starts a new epoch).  g: the particle's
-// unwrapped cell.
-__device__ __forceinline__ void wall_cache_note(const DevParams &p, uint32_t i, float4 q, int3 g)
+// unwrapped cell; stamp: this step's, wc_state[kWcStamp] + 1 before the scan.
+__device__ __forceinline__ void wall_cache_note(const DevParams &p, uint32_t i, float4 q, int3 g, uint32_t stamp)
 {
     if (q.w == (float)CMAG_FLUID) {
         const uint32_t bx = wrap_cell(g.x, p.gx, p.pow2_grid) >> 2, by = wrap_cell(g.y, p.gy, p.pow2_grid) >> 2,
                        bz = wrap_cell(g.z, p.gz, p.pow2_grid) >> 2;
-        p.wc_mark[(bz * p.wc_nby + by) * p.wc_nbx + bx] = p.wc_state[kWcStamp] + 1u;
+        p.wc_mark[(bz * p.wc_nby + by) * p.wc_nbx + bx] = stamp;
     } else {
         const float4 s = p.wc_snap[i];
         if (__float_as_uint(s.x) != __float_as_uint(q.x) || __float_as_uint(s.y) != __float_as_uint(q.y) ||

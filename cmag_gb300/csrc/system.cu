@@ -85,6 +85,11 @@ struct cmag_system {
     bool use_graphs = true;
     cudaGraphExec_t gexec = nullptr;
     bool gvalid = false;
+    // three-launch steps of a small scene: blocks of the cluster (0: staged steps),
+    // decided with the parameters when small_known is false
+    bool small_known = false;
+    uint32_t small_cluster = 0;
+    DevParams small_dev{};
 
     bool timing = false;
     std::vector<cudaEvent_t> events;  // 7 per timed step
@@ -404,6 +409,7 @@ void invalidate_graph(cmag_system *s)
     if (s->gexec) cudaGraphExecDestroy(s->gexec);
     s->gexec = nullptr;
     s->gvalid = false;
+    s->small_known = false;
     verlet_force(s);
     wall_cache_reset(s);
 }
@@ -714,9 +720,32 @@ int capture_graph(cmag_system *s)
     return CMAG_OK;
 }
 
+// Steps of a small planar scene with one lane per particle take three launches
+// (small_step.cu; with or without interaction lists: the list-driven force has the
+// walk's bits).  Staged steps remain for everything else, and where plain stages were
+// asked for (graphs off, stage timing).
+bool small_steps(cmag_system *s)
+{
+    if (!s->use_graphs || s->timing || s->closure || verlet_on(s) || s->g_density != 1 || s->g_force != 1)
+        return false;
+    if (!s->small_known) {
+        s->small_dev = make_dev(s);
+        s->small_cluster = small_step_fits(s->small_dev) ? small_step_cluster(s->small_dev) : 0u;
+        s->small_known = true;
+    }
+    return s->small_cluster != 0;
+}
+
 int do_step(cmag_system *s)
 {
-    if (s->use_graphs && !s->timing && s->stream != nullptr) {
+    if (small_steps(s)) {
+        const bool per = s->p.system == CMAG_PERISTALSIS;
+        const SmallStep a{s->pos, s->vel, s->vlf, s->meas, s->spos, s->svel, per ? s->vforce : s->acc,
+                          per ? s->pforce : nullptr, s->aux, s->hash[0], s->idx[0], s->hash[1], s->idx[1],
+                          s->idx[0], s->cnt, s->off, s->err, s->phase, s->k_milli};
+        CM_CUDA(s, launch_small_step(s->small_dev, a, s->small_cluster, st_of(s)));
+        if (s->vl_flags) verlet_force(s);
+    } else if (s->use_graphs && !s->timing && s->stream != nullptr) {
         if (!s->gvalid) {
             int rc = capture_graph(s);
             if (rc != CMAG_OK) return rc;
@@ -729,6 +758,15 @@ int do_step(cmag_system *s)
     }
     s->last_stage = CMAG_STAGE_INTEGRATE;
     advance_host_mirror(s);
+    return CMAG_OK;
+}
+
+int do_steps(cmag_system *s, uint32_t steps)
+{
+    for (uint32_t k = 0; k < steps; ++k) {
+        int rc = do_step(s);
+        if (rc != CMAG_OK) return rc;
+    }
     return CMAG_OK;
 }
 
@@ -1246,11 +1284,7 @@ int cmag_system_update_dt(cmag_system *s, float dt)
 int cmag_system_update_n(cmag_system *s, uint32_t steps)
 {
     if (!s) return fail(nullptr, CMAG_ERR_INVALID, "null handle");
-    for (uint32_t k = 0; k < steps; ++k) {
-        int rc = do_step(s);
-        if (rc != CMAG_OK) return rc;
-    }
-    return CMAG_OK;
+    return do_steps(s, steps);
 }
 
 int cmag_system_timed_update(cmag_system *s, uint32_t steps, float *ms_out)
@@ -1260,8 +1294,7 @@ int cmag_system_timed_update(cmag_system *s, uint32_t steps, float *ms_out)
     CM_CUDA(s, cudaEventCreate(&a));
     CM_CUDA(s, cudaEventCreate(&b));
     cudaEventRecord(a, st_of(s));
-    int rc = CMAG_OK;
-    for (uint32_t k = 0; k < steps && rc == CMAG_OK; ++k) rc = do_step(s);
+    int rc = do_steps(s, steps);
     cudaEventRecord(b, st_of(s));
     cudaError_t e = cudaEventSynchronize(b);
     float ms = 0.0f;
