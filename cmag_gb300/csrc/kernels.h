@@ -50,34 +50,41 @@ inline int device_sm_count()
 }
 
 // ---- onesweep radix sort (sort.cu) ----------------------------------------
-constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;
-constexpr uint32_t kSortTile = kSortThreads * kSortItems;  // keys per tile
+constexpr int kSortThreads = 1024;
+constexpr uint32_t kSortTiles = 152;  // tiles aimed at: one for each SM of a GB300
 constexpr int kRadixBits = 8;
 constexpr int kRadix = 256;
 constexpr int kMaxPasses = 4;
 
 inline int sort_passes(uint32_t key_bits) { return (int)((key_bits + kRadixBits - 1) / kRadixBits); }
-inline uint32_t sort_tiles(uint32_t n) { return (n + kSortTile - 1) / kSortTile; }
+// Pairs a thread takes (1 to 8): a tile for every SM while that is enough.
+inline uint32_t sort_items(uint32_t n)
+{
+    const uint32_t per = kSortTiles * kSortThreads, items = (n + per - 1) / per;
+    return items < 1 ? 1 : (items > 8 ? 8 : items);
+}
+inline uint32_t sort_tiles(uint32_t n)
+{
+    const uint32_t tile = kSortThreads * sort_items(n);
+    return (n + tile - 1) / tile;
+}
 
 // Workspace of one sort, in 32-bit words: digit histograms [4][256], tile
-// counters [4], then one look-back status array of tiles*256 words per pass.
-// Must be zero when a sort starts (sort_workspace_clear or a memset).
+// counters [4], then one look-back status array per pass (256 words a tile and 256 a
+// group of tiles).
+// Its head (histograms and counters) must be zero when a sort starts.
+size_t sort_head_words();
 size_t sort_workspace_words(uint32_t n, int passes);
 struct SortWorkspace {
     uint32_t *hist;       // [kMaxPasses][256]
     uint32_t *tile_ctr;   // [kMaxPasses]
-    uint32_t *status;     // [passes][tiles][256]
+    uint32_t *status;     // [passes][tiles + groups][256]
 };
 SortWorkspace sort_workspace_view(uint32_t *base, uint32_t n);
 
-// Digit histograms of all passes (used when the hash kernel did not fill them).
-void launch_digit_hist(const uint32_t *keys, uint32_t n, int passes, uint32_t *hist,
-                       cudaStream_t st);
-// One LSD pass on digit `pass`; identity_values: value = input position.
-void launch_onesweep_pass(const uint32_t *kin, const uint32_t *vin, uint32_t *kout,
-                          uint32_t *vout, uint32_t n, int pass, bool identity_values,
-                          const SortWorkspace &ws, uint32_t *err, cudaStream_t st);
+// Stable sort of n pairs on `passes` 8-bit digits; alt_*: n words of scratch each.
+void launch_sort(uint32_t *keys, uint32_t *vals, uint32_t *alt_keys, uint32_t *alt_vals, uint32_t n, int passes,
+                 const SortWorkspace &ws, uint32_t *err, cudaStream_t st);
 
 // ---- cells (cells.cu) --------------------------------------------------------
 // Hash every particle and count particles per cell.  rank (may be null): per

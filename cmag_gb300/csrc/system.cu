@@ -1855,6 +1855,7 @@ namespace {
 struct SortCache {
     uint32_t *ws = nullptr, *keys = nullptr, *vals = nullptr;
     size_t ws_words = 0, cap = 0;
+    uint32_t *err = nullptr;  // host memory the kernels see: failed checks (no copy to read it)
 };
 std::mutex g_sort_mu;
 std::map<int, SortCache> g_sort_cache;
@@ -1873,36 +1874,29 @@ int cmag_sort_particles(uint32_t *d_hash, uint32_t *d_index, uint32_t n, uint32_
     CM_CUDA(nullptr, cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(g_sort_mu);
     SortCache &c = g_sort_cache[dev];
-    const size_t words = sort_workspace_words(n, kMaxPasses) + 1;
+    const size_t words = sort_workspace_words(n, kMaxPasses);
     if (c.cap < n || c.ws_words < words) {
+        const size_t new_words = std::max(c.ws_words, words);
+        const size_t new_cap = std::max(c.cap, (size_t)n);
         if (c.ws) cudaFree(c.ws);
         if (c.keys) cudaFree(c.keys);
         if (c.vals) cudaFree(c.vals);
-        c = SortCache{};
-        CM_CUDA(nullptr, cudaMalloc((void **)&c.ws, words * sizeof(uint32_t)));
-        CM_CUDA(nullptr, cudaMalloc((void **)&c.keys, sizeof(uint32_t) * (size_t)n));
-        CM_CUDA(nullptr, cudaMalloc((void **)&c.vals, sizeof(uint32_t) * (size_t)n));
-        c.ws_words = words;
-        c.cap = n;
+        c.ws = c.keys = c.vals = nullptr;
+        c.ws_words = c.cap = 0;
+        CM_CUDA(nullptr, cudaMalloc((void **)&c.ws, new_words * sizeof(uint32_t)));
+        CM_CUDA(nullptr, cudaMalloc((void **)&c.keys, sizeof(uint32_t) * new_cap));
+        CM_CUDA(nullptr, cudaMalloc((void **)&c.vals, sizeof(uint32_t) * new_cap));
+        c.ws_words = new_words;
+        c.cap = new_cap;
     }
-    uint32_t *err = c.ws + (words - 1);
-    CM_CUDA(nullptr, cudaMemsetAsync(c.ws, 0, words * sizeof(uint32_t), st));
-    SortWorkspace sw = sort_workspace_view(c.ws, n);
-    launch_digit_hist(d_hash, n, passes, sw.hist, st);
-    uint32_t *kb[2] = {d_hash, c.keys}, *vb[2] = {d_index, c.vals};
-    for (int k = 0; k < passes; ++k) {
-        const int src = k & 1, dst = src ^ 1;
-        launch_onesweep_pass(kb[src], vb[src], kb[dst], vb[dst], n, k, false, sw, err, st);
-    }
-    if (passes & 1) {
-        CM_CUDA(nullptr, cudaMemcpyAsync(d_hash, c.keys, sizeof(uint32_t) * (size_t)n,
-                                         cudaMemcpyDeviceToDevice, st));
-        CM_CUDA(nullptr, cudaMemcpyAsync(d_index, c.vals, sizeof(uint32_t) * (size_t)n,
-                                         cudaMemcpyDeviceToDevice, st));
-    }
-    uint32_t bits = 0;
-    CM_CUDA(nullptr, cudaMemcpyAsync(&bits, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    if (!c.err) CM_CUDA(nullptr, cudaHostAlloc((void **)&c.err, sizeof(uint32_t), cudaHostAllocPortable | cudaHostAllocMapped));
+    *c.err = 0;  // (the previous call has waited for its kernels)
+    uint32_t *err = nullptr;
+    CM_CUDA(nullptr, cudaHostGetDevicePointer((void **)&err, c.err, 0));
+    CM_CUDA(nullptr, cudaMemsetAsync(c.ws, 0, sort_head_words() * sizeof(uint32_t), st));
+    launch_sort(d_hash, d_index, c.keys, c.vals, n, passes, sort_workspace_view(c.ws, n), err, st);
     CM_CUDA(nullptr, cudaStreamSynchronize(st));
+    const uint32_t bits = *(volatile uint32_t *)c.err;
     if (bits)
         return fail(nullptr, CMAG_ERR_DEVICE,
                     std::string("sort: device-side check failed (bits ") + std::to_string(bits) + ":" +

@@ -386,7 +386,7 @@ int cmag_sort_particles(uint32_t *d_hash, uint32_t *d_index, uint32_t n, uint32_
  * (a framework's caching allocator, a runtime with a fixed memory budget).  No
  * counterpart in the reference (its thrust::sort_by_key allocates temporaries).
  *  - Works on at most 1,048,576 pairs; larger n returns CMAG_ERR_INVALID.
- *  - Its workspace (about 9.3 MB: look-back status and alternate key/value
+ *  - Its workspace (about 9.1 MB: look-back status and alternate key/value
  *    buffers) is a fixed device array inside this library, held by every GPU that
  *    loads the library until the process exits; no cudaMalloc/cudaFree is called.
  *  - The first call in each CUDA context (normally once per device, in its
