@@ -39,23 +39,25 @@ struct ClosureView {
 // Size of ClosureView::image in 16-byte words.
 uint32_t closure_image_words();
 
+// (nval in the launches below: n float4 of scratch, what the neighbour sums read of a
+// candidate in one load.)
 // Per sorted fluid particle of a DamBreak scene: the 16 raw features, written
 // to feat[idx[i] * 16 ..] (original order).  Rows of wall particles are left
 // untouched.
 void launch_closure_features(const DevParams &p, const float4 *spos, const float4 *svel,
                              const float2 *aux, const float4 *meas, const uint32_t *idx,
-                             const uint32_t *off, const float4 *acc, float *feat,
+                             const uint32_t *off, const float4 *acc, float4 *nval, float *feat,
                              cudaStream_t st);
 // Features (normalised BF16 rows in xb, n x 16, sorted order), network on the
 // tensor cores and acc[idx[i]] += correction for every fluid particle.
 void launch_closure_apply(const DevParams &p, const ClosureView &c, const float4 *spos,
                           const float4 *svel, const float2 *aux, const float4 *meas,
-                          const uint32_t *idx, const uint32_t *off, float4 *acc,
+                          const uint32_t *idx, const uint32_t *off, float4 *acc, float4 *nval,
                           __nv_bfloat16 *xb, cudaStream_t st);
 // Shepard-normalised SPH interpolation of arr (original order) over the fluid
 // particles of a DamBreak scene at n points: out = (value, sum of V_j W).
 void launch_interpolate(const DevParams &p, const float4 *spos, const float2 *aux,
-                        const uint32_t *idx, const uint32_t *off, const float4 *arr,
+                        const uint32_t *idx, const uint32_t *off, const float4 *arr, float4 *nval,
                         const float4 *pts, uint32_t n, float4 *out, cudaStream_t st);
 // Network outputs (unscaled) for n raw feature rows (xb: n x 16 BF16 scratch).
 void launch_closure_forward(const ClosureView &c, const float *feat, uint32_t n,

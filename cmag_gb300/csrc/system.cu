@@ -81,6 +81,7 @@ struct cmag_system {
     bool wc_on = false;
     cmag_closure *closure = nullptr;   // learned correction added after the force stage
     __nv_bfloat16 *closure_x = nullptr;  // its normalised input rows (n x 16)
+    float4 *nval = nullptr;  // scratch of the feature and interpolation walks (n, made on first use)
 
     bool use_graphs = true;
     cudaGraphExec_t gexec = nullptr;
@@ -648,7 +649,7 @@ int record_step(cmag_system *s, int last, bool timed)
                          nullptr, s->phase, nl_of(s), st);
         if (s->closure)
             launch_closure_apply(d, s->closure->view(), s->spos, s->svel, s->aux, s->meas,
-                                 sorted_idx(s), s->off, s->acc, s->closure_x, st);
+                                 sorted_idx(s), s->off, s->acc, s->nval, s->closure_x, st);
     }
     mark(5);
     if (last >= CMAG_STAGE_INTEGRATE)
@@ -795,13 +796,20 @@ void free_all(cmag_system *s)
     void *ptrs[] = {s->pos, s->vel, s->vlf, s->meas, s->acc, s->vforce, s->pforce, s->pred,
                     s->spos, s->svel, s->hash[0], s->hash[1], s->idx[0], s->idx[1], s->cnt,
                     s->off, s->aux, s->ws, s->err, s->phase, s->view_cs, s->view_ce, s->red,
-                    s->zflag, s->closure_x, s->vl_flags, s->vl_xb, s->wc_entry, s->wc_snap,
+                    s->zflag, s->closure_x, s->nval, s->vl_flags, s->vl_xb, s->wc_entry, s->wc_snap,
                     s->wc_mark, s->wc_state};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     free_lists(s);
     if (s->vl_side) cudaStreamDestroy(s->vl_side);
     if (s->own_stream) cudaStreamDestroy(s->own_stream);
+}
+
+// The scratch of the closure's feature and interpolation walks.
+int ensure_nval(cmag_system *s)
+{
+    if (!s->nval) CM_CUDA(s, cudaMalloc((void **)&s->nval, sizeof(float4) * (size_t)s->n));
+    return CMAG_OK;
 }
 
 template <class T>
@@ -991,6 +999,9 @@ int cmag_system_create(const cmag_sph_params *params, uint32_t n, cmag_system **
             }
         }
         s->wc_on = ok;
+        // likewise the interpolation's scratch: when its memory cannot be had now, the
+        // first call that needs it asks again
+        if (rc == CMAG_OK && ensure_nval(s) != CMAG_OK) (void)cudaGetLastError();
     }
     if (rc != CMAG_OK) {
         std::string msg = s->last_error;
@@ -1712,6 +1723,8 @@ int cmag_system_set_closure(cmag_system *s, cmag_closure *c)
     if (!s) return fail(nullptr, CMAG_ERR_INVALID, "null handle");
     if (c && s->p.system != CMAG_DAMBREAK)
         return fail(s, CMAG_ERR_STATE, "the learned closure corrects DamBreak scenes only");
+    if (c)
+        if (int rc = ensure_nval(s)) return rc;
     if (c && !s->closure_x)
         CM_CUDA(s, cudaMalloc((void **)&s->closure_x, sizeof(__nv_bfloat16) * 16 * (size_t)s->n));
     s->closure = c;
@@ -1725,8 +1738,9 @@ int cmag_system_closure_features(cmag_system *s, float *d_features)
     if (s->p.system != CMAG_DAMBREAK) return fail(s, CMAG_ERR_STATE, "not a dam-break system");
     if (s->last_stage < CMAG_STAGE_FORCE)
         return fail(s, CMAG_ERR_STATE, "features need this step's density and forces (run_stages FORCE)");
+    if (int rc = ensure_nval(s)) return rc;
     launch_closure_features(make_dev(s), s->spos, s->svel, s->aux, s->meas, sorted_idx(s), s->off,
-                            s->acc, d_features, st_of(s));
+                            s->acc, s->nval, d_features, st_of(s));
     CM_CUDA(s, cudaGetLastError());
     CM_CUDA(s, cudaStreamSynchronize(st_of(s)));
     return CMAG_OK;
@@ -1747,7 +1761,8 @@ int cmag_system_interpolate(cmag_system *s, int32_t array, const float *d_points
     case CMAG_VELOCITYLEAPFROG: a = s->vlf; break;
     default: return fail(s, CMAG_ERR_INVALID, "not an original-order float4 array: " + std::to_string(array));
     }
-    launch_interpolate(make_dev(s), s->spos, s->aux, sorted_idx(s), s->off, a,
+    if (int rc = ensure_nval(s)) return rc;
+    launch_interpolate(make_dev(s), s->spos, s->aux, sorted_idx(s), s->off, a, s->nval,
                        reinterpret_cast<const float4 *>(d_points), n, reinterpret_cast<float4 *>(d_out),
                        st_of(s));
     CM_CUDA(s, cudaGetLastError());
