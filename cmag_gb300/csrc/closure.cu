@@ -288,19 +288,19 @@ __device__ __forceinline__ uint32_t lds32(const __nv_bfloat16 *p)
 }
 
 // one hidden layer: c[nt] = bias + A x W^T over KT k-tiles; W rows of `stride` BF16
-template <int KT>
+template <int KT, int NT>
 __device__ __forceinline__ void hidden_layer(const __nv_bfloat16 *W, int stride, const float *b,
-                                             const uint32_t (&a)[KT][4], float (&c)[8][4], int g, int t)
+                                             const uint32_t (&a)[KT][4], float (&c)[NT][4], int g, int t)
 {
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
+    for (int nt = 0; nt < NT; ++nt) {
         c[nt][0] = c[nt][2] = b[nt * 8 + 2 * t];
         c[nt][1] = c[nt][3] = b[nt * 8 + 2 * t + 1];
     }
 #pragma unroll
     for (int kt = 0; kt < KT; ++kt)
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
+        for (int nt = 0; nt < NT; ++nt) {
             const __nv_bfloat16 *row = W + (nt * 8 + g) * stride + kt * 16 + 2 * t;
             mma16816(c[nt], a[kt], lds32(row), lds32(row + 8));
         }
@@ -441,20 +441,22 @@ __global__ void __launch_bounds__(128)
 }
 
 // ---- training: forward and backward on the tensor cores ----------------------------
-// A block of 4 warps takes tiles of 64 samples, 16 to a warp.  The forward pass is
-// k_mlp's; each layer's slope of the activation stays in registers, its BF16
-// activations go to shared memory.  The backward products need FP32 deltas against
-// BF16 weights or activations: a delta is split into three BF16 parts (8 + 8 + 8 bits
-// hold its 24) whose products accumulate in FP32, smallest part first, so nothing is
-// rounded that the FP32 form did not round.  Weight gradients (16 rows of each matrix
-// to a warp) accumulate in registers over all of the block's tiles and are added to
-// global memory once.
-// 65,536 samples: 66 us (2.2 M m16n8k16 products), where the form before, 128 samples a
-// block on the FP32 pipes with one 190 KB block an SM, took 423 us; the error against
-// 64 bits is the same (a few 1e-6, activations that round the other way).  Bound by
-// the latency of the chain of layers with two warps a scheduler (255 registers).
+// A block of 8 warps takes tiles of 64 samples; two warps share 16 samples, each with
+// half of a layer's columns.  The forward pass is k_mlp's; each layer's slope of the
+// activation stays in registers, its BF16 activations go to shared memory.  The backward
+// products need FP32 deltas against BF16 weights or activations: a delta is split into
+// three BF16 parts (8 + 8 + 8 bits hold its 24) whose products accumulate in FP32,
+// smallest part first, so nothing is rounded that the FP32 form did not round.  Weight
+// gradients (16 rows and half the columns of each matrix to a warp) accumulate in
+// registers over all of the block's tiles and are added to global memory once.
+// 65,536 samples: 59 us (2.2 M m16n8k16 products); 66 us with one warp to 16 samples (4
+// warps of 255 registers), and 423 us in the form before, 128 samples a block on the
+// FP32 pipes with one 190 KB block an SM.  The error against 64 bits is the same (a few
+// 1e-6: activations that round the other way).  Bound by the chain of layers, five
+// block-wide barriers a tile, at four warps a scheduler, and by the last of four rounds
+// of tiles (1024 over 304 blocks).
 constexpr int kTile = 64;        // samples of a block's tile
-constexpr int kBackThreads = 128;
+constexpr int kBackThreads = 256;  // two warps to 16 samples, 32 of 64 columns each
 constexpr int kXStride = 24;     // BF16 per row of inputs and output deltas (conflict-free)
 constexpr int kHStride = 72;     // BF16 per row of activations and deltas
 constexpr int kPlane = kTile * kHStride;    // one part of a delta
@@ -510,11 +512,12 @@ __device__ __forceinline__ void store_parts(__nv_bfloat16 *at, int plane, float 
 }
 
 // c = activations of a layer (pre-activations in c): BF16 activations of the warp's 16
-// rows to h (row 0 of the warp), slopes to c.
-__device__ __forceinline__ void activate(float (&c)[8][4], __nv_bfloat16 *h, int g, int t)
+// rows to h (its row 0 and first column), slopes to c.
+template <int NT>
+__device__ __forceinline__ void activate(float (&c)[NT][4], __nv_bfloat16 *h, int g, int t)
 {
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
+    for (int nt = 0; nt < NT; ++nt) {
         float a[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -527,9 +530,10 @@ __device__ __forceinline__ void activate(float (&c)[8][4], __nv_bfloat16 *h, int
     }
 }
 
-// c = b + h W^T for the warp's 16 rows (h in shared memory, W rows of kWStride).
+// c = b + h W^T for the warp's 16 rows (h in shared memory; W, b: its first output).
+template <int NT>
 __device__ __forceinline__ void forward_layer(const __nv_bfloat16 *W, const float *b, const __nv_bfloat16 *h,
-                                              float (&c)[8][4], int lane)
+                                              float (&c)[NT][4], int lane)
 {
     const int t = lane & 3, r = lane & 7, q = lane >> 3;
     uint32_t a[4][4];
@@ -537,7 +541,7 @@ __device__ __forceinline__ void forward_layer(const __nv_bfloat16 *W, const floa
     for (int kt = 0; kt < 4; ++kt)
         load_matrices(a[kt], h + (r + (q & 1) * 8) * kHStride + kt * 16 + (q >> 1) * 8);
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
+    for (int nt = 0; nt < NT; ++nt) {
         c[nt][0] = c[nt][2] = b[nt * 8 + 2 * t];
         c[nt][1] = c[nt][3] = b[nt * 8 + 2 * t + 1];
 #pragma unroll
@@ -550,13 +554,15 @@ __device__ __forceinline__ void forward_layer(const __nv_bfloat16 *W, const floa
     }
 }
 
-// c = d W for the warp's 16 rows: the deltas of the layer below before its slopes.
-__device__ __forceinline__ void backward_layer(const __nv_bfloat16 *W, const __nv_bfloat16 *d, float (&c)[8][4],
+// c = d W for the warp's 16 rows (W: its first column): the deltas of the layer below
+// before its slopes.
+template <int NT>
+__device__ __forceinline__ void backward_layer(const __nv_bfloat16 *W, const __nv_bfloat16 *d, float (&c)[NT][4],
                                                int lane)
 {
     const int r = lane & 7, q = lane >> 3;
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.0f;
+    for (int nt = 0; nt < NT; ++nt) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.0f;
 #pragma unroll 1
     for (int part = 2; part >= 0; --part) {
 #pragma unroll
@@ -564,7 +570,7 @@ __device__ __forceinline__ void backward_layer(const __nv_bfloat16 *W, const __n
             uint32_t a[4];
             load_matrices(a, d + part * kPlane + (r + (q & 1) * 8) * kHStride + kt * 16 + (q >> 1) * 8);
 #pragma unroll
-            for (int nt = 0; nt < 8; nt += 2) {
+            for (int nt = 0; nt < NT; nt += 2) {
                 uint32_t w[4];
                 load_matrices_trans(w, W + (kt * 16 + (q & 1) * 8 + r) * kWStride + nt * 8 + (q >> 1) * 8);
                 mma16816(c[nt], a, w[0], w[1]);
@@ -575,13 +581,13 @@ __device__ __forceinline__ void backward_layer(const __nv_bfloat16 *W, const __n
 }
 
 // g[nt] += sum over the tile's samples of d[s][m0 ..] h[s][nt * 8 ..], and the same
-// against ones into gb.  The tile's products are summed from zero, the small parts
+// against ones into gb (bias: in one warp of those that share m0).  The tile's products are summed from zero, the small parts
 // first, and then added: the tensor cores' additions lose up to a unit in the last
 // place of the sum each, always towards zero, which over many tiles shrank the
 // gradient by 8e-7 of it.
 template <int NT, int DSTRIDE, int HSTRIDE>
 __device__ __forceinline__ void weight_grad(float (&g)[NT][4], float (&gb)[4], const __nv_bfloat16 *d, int plane,
-                                            int m0, const __nv_bfloat16 *h, int lane)
+                                            int m0, const __nv_bfloat16 *h, bool bias, int lane)
 {
     constexpr uint32_t kOnes = 0x3f803f80u;
     const int r = lane & 7, q = lane >> 3;
@@ -599,7 +605,7 @@ __device__ __forceinline__ void weight_grad(float (&g)[NT][4], float (&gb)[4], c
                 mma16816(a0[2 * k], a, b[0], b[1]);
                 mma16816(a0[2 * k + 1], a, b[2], b[3]);
             }
-            mma16816(ab, a, kOnes, kOnes);
+            if (bias) mma16816(ab, a, kOnes, kOnes);
         }
     }
 #pragma unroll
@@ -627,11 +633,11 @@ __device__ __forceinline__ void add_gradient(float *grad, int columns, const flo
     }
 }
 
-__device__ __forceinline__ void multiply_store(float (&c)[8][4], const float (&slope)[8][4], __nv_bfloat16 *d, int g,
+__device__ __forceinline__ void multiply_store(float (&c)[4][4], const float (&slope)[4][4], __nv_bfloat16 *d, int g,
                                                int t)
 {
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
+    for (int nt = 0; nt < 4; ++nt) {
         store_parts(d + g * kHStride + nt * 8 + 2 * t, kPlane, c[nt][0] * slope[nt][0], c[nt][1] * slope[nt][1]);
         store_parts(d + (g + 8) * kHStride + nt * 8 + 2 * t, kPlane, c[nt][2] * slope[nt][2], c[nt][3] * slope[nt][3]);
     }
@@ -654,10 +660,14 @@ __global__ void __launch_bounds__(kBackThreads, 2)
     __syncthreads();
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const int w0 = warp * 16;  // the warp's first row in the tile, and its first row of the gradients
+    const int w0 = (warp & 3) * 16;  // the warp's first row in the tile, and its first row of the gradients
+    const int n0 = (warp >> 2) * 32;  // its first column of a layer, and of the gradients
+    const bool left = n0 == 0;
+    auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" : : "r"(1 + (warp & 3)) : "memory"); };
     const float inv_n = 1.0f / (float)n;
-    float g2[8][4] = {}, g3[8][4] = {}, g1[2][4] = {}, g4[2][4] = {};
-    float gb1[4] = {}, gb2[4] = {}, gb3[4] = {}, gb4[4] = {};
+    // ge: W1's gradient in the left warps, W4's in the right ones
+    float g2[4][4] = {}, g3[4][4] = {}, ge[2][4] = {};
+    float gb2[4] = {}, gb3[4] = {}, gbe[4] = {};
     double l = 0.0;
     const uint32_t tiles = (n + kTile - 1) / kTile;
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -673,20 +683,22 @@ __global__ void __launch_bounds__(kBackThreads, 2)
             if (r1 < n) f1 = __ldg(reinterpret_cast<const float2 *>(feat + (size_t)r1 * kFeat + k));
             x[0][2 * half] = pack2((f0.x - m0) * i0, (f0.y - m1) * i1);
             x[0][2 * half + 1] = pack2((f1.x - m0) * i0, (f1.y - m1) * i1);
-            *reinterpret_cast<uint32_t *>(X + (w0 + g) * kXStride + k) = x[0][2 * half];
-            *reinterpret_cast<uint32_t *>(X + (w0 + g + 8) * kXStride + k) = x[0][2 * half + 1];
+            if (left) {
+                *reinterpret_cast<uint32_t *>(X + (w0 + g) * kXStride + k) = x[0][2 * half];
+                *reinterpret_cast<uint32_t *>(X + (w0 + g + 8) * kXStride + k) = x[0][2 * half + 1];
+            }
         }
         // forward
-        float s1[8][4], s2[8][4], c[8][4];
-        hidden_layer<1>(sw + kSW1, kW1Stride, sb + kSB1, x, s1, g, t);
-        activate(s1, H1 + w0 * kHStride, g, t);
-        __syncwarp();
-        forward_layer(sw + kSW2, sb + kSB2, H1 + w0 * kHStride, s2, lane);
-        activate(s2, H2 + w0 * kHStride, g, t);
-        __syncwarp();
-        forward_layer(sw + kSW3, sb + kSB3, H2 + w0 * kHStride, c, lane);
-        activate(c, H3 + w0 * kHStride, g, t);
-        __syncwarp();
+        float s1[4][4], s2[4][4], c[4][4];
+        hidden_layer<1>(sw + kSW1 + n0 * kW1Stride, kW1Stride, sb + kSB1 + n0, x, s1, g, t);
+        activate(s1, H1 + w0 * kHStride + n0, g, t);
+        pair_sync();
+        forward_layer(sw + kSW2 + n0 * kWStride, sb + kSB2 + n0, H1 + w0 * kHStride, s2, lane);
+        activate(s2, H2 + w0 * kHStride + n0, g, t);
+        pair_sync();
+        forward_layer(sw + kSW3 + n0 * kWStride, sb + kSB3 + n0, H2 + w0 * kHStride, c, lane);
+        activate(c, H3 + w0 * kHStride + n0, g, t);
+        pair_sync();
         // outputs, in FP32 (three columns: a lane's 16 activations of each row, then the
         // four lanes of the row), and the output deltas
         float d0[kOut], d1[kOut];
@@ -708,61 +720,61 @@ __global__ void __launch_bounds__(kBackThreads, 2)
             const float b = sb[kSB4 + o];
             d0[o] = r0 < n ? y0 + b - __ldg(target + (size_t)r0 * kOut + o) : 0.0f;
             d1[o] = r1 < n ? y1 + b - __ldg(target + (size_t)r1 * kOut + o) : 0.0f;
-            if (t == 0) l += (double)d0[o] * d0[o] + (double)d1[o] * d1[o];
+            if (left && t == 0) l += (double)d0[o] * d0[o] + (double)d1[o] * d1[o];
             d0[o] *= inv_n;
             d1[o] *= inv_n;
         }
-        if (t == 0) {
+        if (left && t == 0) {
             store_parts(D4 + (w0 + g) * kXStride, kPlane4, d0[0], d0[1]);
             store_parts(D4 + (w0 + g + 8) * kXStride, kPlane4, d1[0], d1[1]);
-        } else if (t == 1) {
+        } else if (left && t == 1) {
             store_parts(D4 + (w0 + g) * kXStride + 2, kPlane4, d0[2], 0.0f);
             store_parts(D4 + (w0 + g + 8) * kXStride + 2, kPlane4, d1[2], 0.0f);
         }
         // layer 3's deltas (W4 has three rows: FP32)
-        float d[8][4];
+        float d[4][4];
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
+        for (int nt = 0; nt < 4; ++nt) {
             d[nt][0] = d[nt][1] = d[nt][2] = d[nt][3] = 0.0f;
 #pragma unroll
             for (int o = 0; o < kOut; ++o) {
-                const float2 w = unpack2(lds32(sw + kSW4 + o * kWStride + nt * 8 + 2 * t));
+                const float2 w = unpack2(lds32(sw + kSW4 + o * kWStride + n0 + nt * 8 + 2 * t));
                 d[nt][0] = __fmaf_rn(w.x, d0[o], d[nt][0]);
                 d[nt][1] = __fmaf_rn(w.y, d0[o], d[nt][1]);
                 d[nt][2] = __fmaf_rn(w.x, d1[o], d[nt][2]);
                 d[nt][3] = __fmaf_rn(w.y, d1[o], d[nt][3]);
             }
         }
-        multiply_store(d, c, D + w0 * kHStride, g, t);
+        multiply_store(d, c, D + w0 * kHStride + n0, g, t);
         __syncthreads();
-        weight_grad<2, kXStride, kHStride>(g4, gb4, D4, kPlane4, 0, H3 + w0, lane);
-        weight_grad<8, kHStride, kHStride>(g3, gb3, D, kPlane, w0, H2, lane);
-        backward_layer(sw + kSW3, D + w0 * kHStride, c, lane);
+        if (!left) weight_grad<2, kXStride, kHStride>(ge, gbe, D4, kPlane4, 0, H3 + w0, true, lane);
+        weight_grad<4, kHStride, kHStride>(g3, gb3, D, kPlane, w0, H2 + n0, left, lane);
+        backward_layer(sw + kSW3 + n0, D + w0 * kHStride, c, lane);
         __syncthreads();
-        multiply_store(c, s2, D + w0 * kHStride, g, t);
+        multiply_store(c, s2, D + w0 * kHStride + n0, g, t);
         __syncthreads();
-        weight_grad<8, kHStride, kHStride>(g2, gb2, D, kPlane, w0, H1, lane);
-        backward_layer(sw + kSW2, D + w0 * kHStride, c, lane);
+        weight_grad<4, kHStride, kHStride>(g2, gb2, D, kPlane, w0, H1 + n0, left, lane);
+        backward_layer(sw + kSW2 + n0, D + w0 * kHStride, c, lane);
         __syncthreads();
-        multiply_store(c, s1, D + w0 * kHStride, g, t);
+        multiply_store(c, s1, D + w0 * kHStride + n0, g, t);
         __syncthreads();
-        weight_grad<2, kHStride, kXStride>(g1, gb1, D, kPlane, w0, X, lane);
+        if (left) weight_grad<2, kHStride, kXStride>(ge, gbe, D, kPlane, w0, X, true, lane);
         __syncthreads();
     }
-    add_gradient(grad + kOffW1, kFeat, g1, w0 + g, kHidden, 0, t);
-    add_gradient(grad + kOffW2, kHidden, g2, w0 + g, kHidden, 0, t);
-    add_gradient(grad + kOffW3, kHidden, g3, w0 + g, kHidden, 0, t);
-    add_gradient(grad + kOffW4, kHidden, g4, g, kOut, w0, t);
-    if (t == 0) {  // every column of a bias product holds the sum
+    add_gradient(grad + kOffW2, kHidden, g2, w0 + g, kHidden, n0, t);
+    add_gradient(grad + kOffW3, kHidden, g3, w0 + g, kHidden, n0, t);
+    if (left) add_gradient(grad + kOffW1, kFeat, ge, w0 + g, kHidden, 0, t);
+    else add_gradient(grad + kOffW4, kHidden, ge, g, kOut, w0, t);
+    if (t == 0 && left) {  // every column of a bias product holds the sum
         const int o = w0 + g;
-        atomicAdd(grad + kOffB1 + o, gb1[0]);
-        atomicAdd(grad + kOffB1 + o + 8, gb1[2]);
+        atomicAdd(grad + kOffB1 + o, gbe[0]);
+        atomicAdd(grad + kOffB1 + o + 8, gbe[2]);
         atomicAdd(grad + kOffB2 + o, gb2[0]);
         atomicAdd(grad + kOffB2 + o + 8, gb2[2]);
         atomicAdd(grad + kOffB3 + o, gb3[0]);
         atomicAdd(grad + kOffB3 + o + 8, gb3[2]);
-        if (warp == 0 && g < kOut) atomicAdd(grad + kOffB4 + g, gb4[0]);
     }
+    if (t == 0 && warp == 4 && g < kOut) atomicAdd(grad + kOffB4 + g, gbe[0]);
 #pragma unroll
     for (int w = 16; w > 0; w >>= 1) l += __shfl_xor_sync(0xffffffffu, l, w);
     // FP64: few operations, and the sum of many small squares keeps its digits
