@@ -81,7 +81,9 @@ struct cmag_system {
     bool wc_on = false;
     cmag_closure *closure = nullptr;   // learned correction added after the force stage
     __nv_bfloat16 *closure_x = nullptr;  // its normalised input rows (n x 16)
-    float4 *nval = nullptr;  // scratch of the feature and interpolation walks (n, made on first use)
+    // scratch of the feature and interpolation walks (n): behind wc_snap, or made on first use
+    float4 *nval = nullptr;
+    bool nval_own = false;
 
     bool use_graphs = true;
     cudaGraphExec_t gexec = nullptr;
@@ -796,7 +798,7 @@ void free_all(cmag_system *s)
     void *ptrs[] = {s->pos, s->vel, s->vlf, s->meas, s->acc, s->vforce, s->pforce, s->pred,
                     s->spos, s->svel, s->hash[0], s->hash[1], s->idx[0], s->idx[1], s->cnt,
                     s->off, s->aux, s->ws, s->err, s->phase, s->view_cs, s->view_ce, s->red,
-                    s->zflag, s->closure_x, s->nval, s->vl_flags, s->vl_xb, s->wc_entry, s->wc_snap,
+                    s->zflag, s->closure_x, s->nval_own ? s->nval : nullptr, s->vl_flags, s->vl_xb, s->wc_entry, s->wc_snap,
                     s->wc_mark, s->wc_state};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -808,7 +810,9 @@ void free_all(cmag_system *s)
 // The scratch of the closure's feature and interpolation walks.
 int ensure_nval(cmag_system *s)
 {
-    if (!s->nval) CM_CUDA(s, cudaMalloc((void **)&s->nval, sizeof(float4) * (size_t)s->n));
+    if (s->nval) return CMAG_OK;
+    CM_CUDA(s, cudaMalloc((void **)&s->nval, sizeof(float4) * (size_t)s->n));
+    s->nval_own = true;
     return CMAG_OK;
 }
 
@@ -987,7 +991,7 @@ int cmag_system_create(const cmag_sph_params *params, uint32_t n, cmag_system **
         for (int a = 0; a < 3; ++a) s->wc_nb[a] = (params->grid_size[a] + 3u) / 4u;
         const size_t marks = sizeof(uint32_t) * (size_t)s->wc_nb[0] * s->wc_nb[1] * s->wc_nb[2];
         void **bufs[4] = {(void **)&s->wc_entry, (void **)&s->wc_snap, (void **)&s->wc_mark, (void **)&s->wc_state};
-        const size_t sizes[4] = {f4, f4, marks, 4 * sizeof(uint32_t)};
+        const size_t sizes[4] = {f4, 2 * f4, marks, 4 * sizeof(uint32_t)};  // snapshots, then nval
         bool ok = true;
         for (int k = 0; k < 4 && ok; ++k)
             ok = cudaMalloc(bufs[k], sizes[k]) == cudaSuccess && cudaMemset(*bufs[k], 0, sizes[k]) == cudaSuccess;
@@ -999,9 +1003,7 @@ int cmag_system_create(const cmag_sph_params *params, uint32_t n, cmag_system **
             }
         }
         s->wc_on = ok;
-        // likewise the interpolation's scratch: when its memory cannot be had now, the
-        // first call that needs it asks again
-        if (rc == CMAG_OK && ensure_nval(s) != CMAG_OK) (void)cudaGetLastError();
+        if (ok) s->nval = s->wc_snap + n;
     }
     if (rc != CMAG_OK) {
         std::string msg = s->last_error;
