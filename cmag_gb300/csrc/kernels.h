@@ -181,6 +181,11 @@ void launch_verlet_check(const float4 *pos, const float4 *xb, uint32_t start, ui
 // solvers in turn, us per step of each, here / staged: 352 particles 6.2 / 15.7,
 // 3,840 11 / 21, 16,384 20.5 / 23.8, 21,200 22.3 / 19.8, 34,800 33 / 21.
 constexpr uint32_t kSmallParticles = 18000;
+// Up to here the three launches also beat the staged step at the lanes the autotuner
+// finds (us a step of one solver, three launches / tuned stages: Poiseuille 4480
+// particles 20.0 / 28.7, dam break 8702 31.3 / 43.7, 16,918 44.8 / 37.9, Peristalsis
+// 16,384 41.0 / 35.9).
+constexpr uint32_t kSmallTuned = 10000;
 constexpr uint32_t kSmallCells = 1u << 18;  // the sort's cluster scans them in a few us
 // The arrays of launch_hash .. launch_integrate; rank may alias idx.
 struct SmallStep {

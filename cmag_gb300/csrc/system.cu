@@ -727,10 +727,9 @@ int capture_graph(cmag_system *s)
 // (small_step.cu; with or without interaction lists: the list-driven force has the
 // walk's bits).  Staged steps remain for everything else, and where plain stages were
 // asked for (graphs off, stage timing).
-bool small_steps(cmag_system *s)
+bool small_form(cmag_system *s)  // whatever the lanes
 {
-    if (!s->use_graphs || s->timing || s->closure || verlet_on(s) || s->g_density != 1 || s->g_force != 1)
-        return false;
+    if (!s->use_graphs || s->timing || s->closure || verlet_on(s)) return false;
     if (!s->small_known) {
         s->small_dev = make_dev(s);
         s->small_cluster = small_step_fits(s->small_dev) ? small_step_cluster(s->small_dev) : 0u;
@@ -738,6 +737,7 @@ bool small_steps(cmag_system *s)
     }
     return s->small_cluster != 0;
 }
+bool small_steps(cmag_system *s) { return s->g_density == 1 && s->g_force == 1 && small_form(s); }
 
 int do_step(cmag_system *s)
 {
@@ -1626,6 +1626,13 @@ int cmag_system_autotune(cmag_system *s, int32_t reps)
         if (!lists) free_lists(s);
     } else if (had_lists) {
         (void)cudaGetLastError();
+    }
+    // the trials time staged kernels; up to kSmallTuned particles a step of three
+    // launches, which takes one lane, beats the best of them
+    if (s->n <= kSmallTuned && small_form(s)) {
+        gd = gf = 1;
+        if (lists) free_lists(s);
+        lists = false;
     }
     s->last_error.clear();
     cudaEventDestroy(a);

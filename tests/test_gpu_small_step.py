@@ -117,3 +117,23 @@ def test_three_launch_steps_equal_staged_steps(gpu, name, lists):
     x, y = a.state(), b.state()
     for k in x:
         assert np.array_equal(x[k].view(np.uint32), y[k].view(np.uint32)), (name, k)
+
+
+@pytest.mark.parametrize("make,one_lane", [(lambda: poiseuille(64, 64), True), (lambda: dambreak(64), True),
+                                           (lambda: poiseuille(160, 100), None)])
+def test_autotuned_scene(gpu, make, one_lane):
+    """The autotuner keeps one lane where the three launches are the fastest step, and
+    what it then steps has the untuned system's bits."""
+    a, b = make(), make()
+    for s in (a, b):
+        jittered(s, 4)
+    lanes = tuple(b.autotune(2))
+    if one_lane:
+        assert lanes == (1, 1, False)
+    a.update_n(20)
+    b.update_n(20)
+    if lanes == (1, 1, False):
+        for array in (cm.POSITION, cm.VELOCITY, cm.MEASURES):
+            assert np.array_equal(a.getArray(array), b.getArray(array))
+    a.close()
+    b.close()
