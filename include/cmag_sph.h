@@ -303,7 +303,8 @@ int cmag_system_fluid_sum(cmag_system *s, int32_t array, double sum[4], uint32_t
 /* Use a caller-owned cudaStream_t (NULL = the instance's own stream). */
 int cmag_system_set_stream(cmag_system *s, void *cuda_stream);
 void *cmag_system_stream(const cmag_system *s);
-/* 1: capture each step as a CUDA graph and replay it (default); 0: plain launches. */
+/* 1: capture each step as a CUDA graph and replay it (default; planar scenes of up to
+ * 18,000 particles at one lane launch three kernels a step directly); 0: plain launches. */
 int cmag_system_set_graphs(cmag_system *s, int32_t enable);
 /* Wait for the instance's stream and report device-side check failures
  * (CMAG_ERR_DEVICE with the cmag_device_error bits in the message). */
@@ -327,10 +328,9 @@ int cmag_system_get_neighbor_lists(const cmag_system *s, int32_t *enabled, uint3
  * same non-fluid particles in the same order, so the reused value has the bits
  * the walk would give).  A non-fluid particle that moves or changes type, and any
  * change of parameters, lanes or lists, starts over.  On by default for DamBreak
- * (memory: num_particles x 48 bytes, 16 of them scratch of the
- * interpolation, + 4 bytes per 4x4x4 cells; an instance whose
- * creation could not have that memory is made without it); other families have
- * nothing to keep.  enable = 1 without kept wall densities: CMAG_ERR_STATE. */
+ * (memory: num_particles x 48 bytes, 16 of them scratch of the interpolation, + 4
+ * bytes per 4x4x4 cells; an instance whose creation could not have that memory is
+ * made without it); other families have nothing to keep.  enable = 1 without kept wall densities: CMAG_ERR_STATE. */
 int cmag_system_set_wall_cache(cmag_system *s, int32_t enable);
 int cmag_system_get_wall_cache(const cmag_system *s, int32_t *enabled);
 /* Neighbour lists kept over several steps.  No counterpart in the reference,
@@ -358,7 +358,8 @@ int cmag_system_set_verlet(cmag_system *s, float skin);
 int cmag_system_get_verlet(cmag_system *s, float *skin, uint32_t *rebuilds);
 /* Autotune: on the current state, time the density and force kernels for every
  * lane count and with interaction lists (`reps` launches each) and keep the
- * fastest.  Both kernels are recomputed from scratch every step; the choice
+ * fastest (planar scenes of up to 10,000 particles keep one lane, whose step of three
+ * launches is faster).  Both kernels are recomputed from scratch every step; the choice
  * changes only the summation order of the lanes' partial sums. */
 int cmag_system_autotune(cmag_system *s, int32_t reps);
 
