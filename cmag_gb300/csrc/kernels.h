@@ -176,10 +176,10 @@ void launch_verlet_check(const float4 *pos, const float4 *xb, uint32_t start, ui
                          uint32_t *moved, cudaStream_t st);
 
 // ---- the step of a small planar scene in three launches (small_step.cu) ----------
-// Largest scene that takes it.  The neighbour loops' 8 lanes cost several times the
+// Largest scene that takes it.  The neighbour loops' lanes cost several times the
 // instructions of one lane, which pays while the GPU has idle issue slots: three
 // solvers in turn, us per step of each, here / staged: 352 particles 6.2 / 15.7,
-// 3,840 11 / 21, 16,384 20.5 / 23.8, 21,200 22.3 / 19.8, 34,800 33 / 21.
+// 3,840 11 / 21, 16,384 18.6 / 23.8; with 8 lanes 21,200 22.3 / 19.8, 34,800 33 / 21.
 constexpr uint32_t kSmallParticles = 18000;
 // Up to here the three launches also beat the staged step at the lanes the autotuner
 // finds (us a step of one solver, three launches / tuned stages: Poiseuille 4480

@@ -11,13 +11,14 @@
 //     distributed shared memory.  Bound by the latency of its five stages (10-17 us).
 //     512 threads a block: at 1024 the cluster waits for 16 SMs that are nearly empty
 //     when other solvers run beside it (20.5 against 25 us a step, 16,384 particles);
-//   * the density and the force give each particle 8 lanes, one per row of its cell
-//     box, so a particle's cell lookups and loads are in flight together.  Bound by
-//     that latency up to about 10,000 particles, then by instruction issue;
+//   * the density and the force give each particle 8 lanes (4 in the larger scenes),
+//     one per row of its cell box, so a particle's cell lookups and loads are in
+//     flight together.  Bound by that latency up to about 10,000 particles, then by
+//     instruction issue;
 //   * the force launch integrates its particles too.
 // One solver alone, us per step: Poiseuille 4,480 particles 41 -> 20.5, dam break
-// 8,702 61 -> 32, Peristalsis 16,384 58.5 -> 39; three solvers in turn, where the
-// host's 15 us a step counts: 16.5 -> 8.5, 37.8 -> 31.7, 23.8 -> 20.5.
+// 8,702 61 -> 32, Peristalsis 16,384 58.5 -> 43; three solvers in turn, where the
+// host's 15 us a step counts: 16.5 -> 8.5, 37.8 -> 31.7, 23.8 -> 18.6.
 //
 // Same bits as the staged step with one lane per particle: the lanes leave their
 // candidates' terms in shared memory, and one lane per sum adds them in the order of
@@ -167,17 +168,25 @@ __global__ void __launch_bounds__(kSortBlock, 1) k_small_sort(DevParams p, Small
     }
 }
 
-// ---- neighbour loops: 8 lanes per particle, lane r on row r of its cell box ----------
+// ---- neighbour loops: L lanes per particle, lane r on row r of a batch of L rows ------
 
-constexpr int kLanes = 8;
+// 8 lanes take a box of 7 rows at once: the shortest chain, and the form of scenes up to
+// kWideParticles.  4 lanes take it in two batches with half the warps: above that line,
+// where solvers that share the GPU compete for issue slots (us per step of each of three
+// solvers, 8 lanes / 4: 4480 particles 8.5 / 10.4, 8702 15.0 / 16.3, 16,384 20.5 / 18.6,
+// 16,960 21.0 / 17.9; one solver alone 19.6 / 29.2, 31.3 / 38.4, 41.0 / 43.6, 34.8 / 33.1).
+constexpr uint32_t kWideParticles = 12000;
 constexpr int kSlots = 8;            // terms of a row held at once
 constexpr uint32_t kRowMost = 32;    // candidates of a row that one lane takes
-constexpr int kLoopThreads = 256;    // per block: 32 particles
-constexpr int kGroups = 32 / kLanes; // particles of a warp
+constexpr int kLoopThreads = 256;    // per block
 // Words between the slots of neighbouring rows: `words` for each of the warp's
 // particles and as many of padding, so that the lanes that write a slot, and those
 // that read one, fall into different banks.
-__host__ __device__ constexpr int slot_stride(int words) { return words * (kGroups + 1); }
+template <int L>
+__host__ __device__ constexpr int slot_stride(int words)
+{
+    return words * (32 / L + 1);
+}
 
 // The candidates of one row: sorted particles b0, b0 + 1, ... (n0 of them) and, when
 // the row wraps in x, n1 more from b1; with their image shifts.
@@ -205,20 +214,21 @@ __device__ __forceinline__ Row find_row(const DevParams &p, const uint32_t *off,
 }
 
 // Lanes of one particle.
+template <int L>
 struct Group {
     uint32_t mask;
     int lane, index;
     __device__ __forceinline__ Group()
     {
         const int l = threadIdx.x & 31;
-        lane = l % kLanes;
-        index = l / kLanes;
-        mask = ((1u << kLanes) - 1u) << (l - lane);
+        lane = l % L;
+        index = l / L;
+        mask = ((1u << L) - 1u) << (l - lane);
     }
     template <class T>
     __device__ __forceinline__ T get(T v, int from) const
     {
-        return __shfl_sync(mask, v, from, kLanes);
+        return __shfl_sync(mask, v, from, L);
     }
     __device__ __forceinline__ Row get(const Row &v, int from) const
     {
@@ -231,7 +241,7 @@ struct Group {
     // first of the particle's `words` words of slot k of row r
     __device__ __forceinline__ int slot(int k, int r, int words) const
     {
-        return (k * kLanes + r) * slot_stride(words) + index * words;
+        return (k * L + r) * slot_stride<L>(words) + index * words;
     }
 };
 
@@ -270,8 +280,8 @@ __device__ __forceinline__ float spline_weight(const DevParams &p, float4 pi, fl
 
 // Lanes 0 .. lanes - 1 add the rows' slots in order, K slots a row (the row's `at`
 // terms and exact zeros).
-template <int K>
-__device__ __forceinline__ void sum_slots(const Group &gr, float *s, uint32_t at, int lanes, float &sum)
+template <int K, int L>
+__device__ __forceinline__ void sum_slots(const Group<L> &gr, float *s, uint32_t at, int lanes, float &sum)
 {
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -279,7 +289,7 @@ __device__ __forceinline__ void sum_slots(const Group &gr, float *s, uint32_t at
     gr.sync();
     if (gr.lane < lanes) {
 #pragma unroll
-        for (int r = 0; r < kLanes; ++r)
+        for (int r = 0; r < L; ++r)
 #pragma unroll
             for (int k = 0; k < K; ++k) {
                 const float2 v = *reinterpret_cast<const float2 *>(s + gr.slot(k, r, 4) + 2 * gr.lane);
@@ -294,8 +304,8 @@ __device__ __forceinline__ void sum_slots(const Group &gr, float *s, uint32_t at
 // ones; cubic spline: lane 0 adds all.  Each lane leaves its row's non-zero terms in
 // its slots, then they are added row by row.  For rows of at most kRowMost candidates;
 // false (and nothing added) when a row has more terms than slots.
-template <int SYS>
-__device__ __forceinline__ bool add_rows(const DevParams &p, const float4 *spos, const Group &gr, const Row &row,
+template <int SYS, int L>
+__device__ __forceinline__ bool add_rows(const DevParams &p, const float4 *spos, const Group<L> &gr, const Row &row,
                                          float4 pi, float *s, float &sum)
 {
     // a term is stored behind the row's earlier ones and counted when it is not zero
@@ -356,18 +366,18 @@ __device__ __forceinline__ bool add_rows(const DevParams &p, const float4 *spos,
 
 // The same with rows of any length, one after another, every lane on the row's next
 // candidates (pair steps).
-template <int SYS>
-__device__ __noinline__ float add_long_rows(const DevParams &p, const float4 *spos, const Group &gr, const Row &mine,
+template <int SYS, int L>
+__device__ __noinline__ float add_long_rows(const DevParams &p, const float4 *spos, const Group<L> &gr, const Row &mine,
                                             float4 pi, float *s, float sum)
 {
     const bool wendland = p.kernel == CMAG_KERNEL_WENDLAND;
     const uint32_t per = wendland ? 2u : 1u;  // candidates a lane takes
-    for (int r = 0; r < kLanes; ++r) {
+    for (int r = 0; r < L; ++r) {
         const Row row = gr.get(mine, r);
         for (int part = 0; part < 2; ++part) {
             const uint32_t b = part ? row.b1 : row.b0, e = b + (part ? row.n1 : row.n0);
             const float sx = part ? row.sx1 : row.sx0;
-            for (uint32_t base = b; base < e; base += per * kLanes) {
+            for (uint32_t base = b; base < e; base += per * L) {
                 const uint32_t j = base + per * gr.lane;
                 float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 if (j < e) {
@@ -383,7 +393,7 @@ __device__ __noinline__ float add_long_rows(const DevParams &p, const float4 *sp
                 *reinterpret_cast<float4 *>(s + gr.slot(0, gr.lane, 4)) = w;
                 gr.sync();
                 if (gr.lane < (int)per) {
-                    for (int l = 0; l < kLanes; ++l) {
+                    for (int l = 0; l < L; ++l) {
                         const float2 v = *reinterpret_cast<const float2 *>(s + gr.slot(0, l, 4) + 2 * gr.lane);
                         sum = __fmaf_rn(v.x, v.y, sum);
                     }
@@ -396,14 +406,14 @@ __device__ __noinline__ float add_long_rows(const DevParams &p, const float4 *sp
 }
 
 // Density (k_density).
-template <int SYS, bool TRIM>
+template <int SYS, bool TRIM, int L>
 __global__ void __launch_bounds__(kLoopThreads, 4) k_small_density(DevParams p, SmallStep a)
 {
     pdl_entry();
-    __shared__ float4 s_all[kLoopThreads / 32][(kSlots + 1) * kLanes * slot_stride(4) / 4];
+    __shared__ float4 s_all[kLoopThreads / 32][(kSlots + 1) * L * slot_stride<L>(4) / 4];
     float *const s = reinterpret_cast<float *>(s_all[threadIdx.x >> 5]);
-    const Group gr;
-    const uint32_t i = (blockIdx.x * kLoopThreads + threadIdx.x) / kLanes;
+    const Group<L> gr;
+    const uint32_t i = (blockIdx.x * kLoopThreads + threadIdx.x) / L;
     if (i >= p.n) return;  // whole groups
     const float4 pi = __ldg(a.spos + i);
     const bool pinned = SYS == CMAG_POISEUILLE && pi.w == 1.0f;
@@ -418,7 +428,7 @@ __global__ void __launch_bounds__(kLoopThreads, 4) k_small_density(DevParams p, 
     if (!pinned && wc != 2u) {
         const float3 f = walk::frac_cell(p, pi);
         const bool wendland = p.kernel == CMAG_KERNEL_WENDLAND;
-        for (int dy0 = -p.cell_count; dy0 <= p.cell_count; dy0 += kLanes) {
+        for (int dy0 = -p.cell_count; dy0 <= p.cell_count; dy0 += L) {
             const Row row = find_row<SYS, TRIM>(p, a.off, dy0 + gr.lane, g, f);
             if (!gr.all(row.n0 + row.n1 <= kRowMost) || !add_rows<SYS>(p, a.spos, gr, row, pi, s, sum))
                 sum = add_long_rows<SYS>(p, a.spos, gr, row, pi, s, sum);
@@ -476,8 +486,8 @@ struct Slot {
         }
     }
     // like sum_slots
-    template <int K>
-    static __device__ __forceinline__ void add(const Group &gr, float *s, uint32_t at, float &sum)
+    template <int K, int L>
+    static __device__ __forceinline__ void add(const Group<L> &gr, float *s, uint32_t at, float &sum)
     {
 #pragma unroll
         for (int k = 0; k < K; ++k)
@@ -485,7 +495,7 @@ struct Slot {
         gr.sync();
         if (gr.lane < lanes) {
 #pragma unroll
-            for (int r = 0; r < kLanes; ++r)
+            for (int r = 0; r < L; ++r)
 #pragma unroll
                 for (int k = 0; k < K; ++k) take(s + gr.slot(k, r, words), gr.lane, sum);
         }
@@ -494,8 +504,8 @@ struct Slot {
 };
 
 // The force sums over the rows of one batch, like add_rows and add_long_rows.
-template <int SYS, bool TRIM>
-__device__ __forceinline__ bool add_row_forces(const DevParams &p, const SmallStep &a, const Group &gr,
+template <int SYS, bool TRIM, int L>
+__device__ __forceinline__ bool add_row_forces(const DevParams &p, const SmallStep &a, const Group<L> &gr,
                                                const Row &row, const PairSelf &self, float *s, float &sum)
 {
     constexpr uint32_t U = 4;  // candidates loaded together
@@ -532,16 +542,16 @@ __device__ __forceinline__ bool add_row_forces(const DevParams &p, const SmallSt
     return true;
 }
 
-template <int SYS, bool TRIM>
-__device__ __noinline__ float add_long_row_forces(const DevParams &p, const SmallStep &a, const Group &gr,
+template <int SYS, bool TRIM, int L>
+__device__ __noinline__ float add_long_row_forces(const DevParams &p, const SmallStep &a, const Group<L> &gr,
                                                   const Row &mine, const PairSelf &self, float *s, float sum)
 {
-    for (int r = 0; r < kLanes; ++r) {
+    for (int r = 0; r < L; ++r) {
         const Row row = gr.get(mine, r);
         for (int part = 0; part < 2; ++part) {
             const uint32_t b = part ? row.b1 : row.b0, e = b + (part ? row.n1 : row.n0);
             const float sx = part ? row.sx1 : row.sx0;
-            for (uint32_t base = b; base < e; base += kLanes) {
+            for (uint32_t base = b; base < e; base += L) {
                 const uint32_t j = base + gr.lane < e ? base + gr.lane : self.i;
                 PairTerms t{};
                 const float4 q = __ldg(a.spos + j);
@@ -552,7 +562,7 @@ __device__ __noinline__ float add_long_row_forces(const DevParams &p, const Smal
                 Slot<SYS>::put(s + gr.slot(0, gr.lane, Slot<SYS>::words), t);
                 gr.sync();
                 if (gr.lane < Slot<SYS>::lanes)
-                    for (int l = 0; l < kLanes; ++l)
+                    for (int l = 0; l < L; ++l)
                         Slot<SYS>::take(s + gr.slot(0, l, Slot<SYS>::words), gr.lane, sum);
                 gr.sync();
             }
@@ -562,15 +572,15 @@ __device__ __noinline__ float add_long_row_forces(const DevParams &p, const Smal
 }
 
 // Force (k_force) and integration (k_integrate) of the same particle.
-template <int SYS, bool TRIM>
+template <int SYS, bool TRIM, int L>
 __global__ void __launch_bounds__(kLoopThreads, 2) k_small_force(DevParams p, SmallStep a)
 {
     pdl_entry();
     extern __shared__ float4 smem[];
-    constexpr int kWords = (Slot<SYS>::count + 1) * kLanes * slot_stride(Slot<SYS>::words);  // of a warp
+    constexpr int kWords = (Slot<SYS>::count + 1) * L * slot_stride<L>(Slot<SYS>::words);  // of a warp
     float *const s = reinterpret_cast<float *>(smem) + (threadIdx.x >> 5) * kWords;
-    const Group gr;
-    const uint32_t i = (blockIdx.x * kLoopThreads + threadIdx.x) / kLanes;
+    const Group<L> gr;
+    const uint32_t i = (blockIdx.x * kLoopThreads + threadIdx.x) / L;
     if (i >= p.n) return;  // whole groups
     float4 pi = __ldg(a.spos + i);
     if (SYS == CMAG_DAMBREAK && pi.w != (float)CMAG_FLUID) return;
@@ -580,7 +590,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_small_force(DevParams p, Sm
     const int3 g = grid_pos(p, pi.x, pi.y, pi.z);
     const float3 f = walk::frac_cell(p, pi);
     float sum = 0.0f;
-    for (int dy0 = -p.cell_count; dy0 <= p.cell_count; dy0 += kLanes) {
+    for (int dy0 = -p.cell_count; dy0 <= p.cell_count; dy0 += L) {
         const Row row = find_row<SYS, TRIM>(p, a.off, dy0 + gr.lane, g, f);
         if (!gr.all(row.n0 + row.n1 <= kRowMost) || !add_row_forces<SYS, TRIM>(p, a, gr, row, self, s, sum))
             sum = add_long_row_forces<SYS, TRIM>(p, a, gr, row, self, s, sum);
@@ -615,20 +625,29 @@ using SmallKernel = void (*)(DevParams, SmallStep);
 
 struct Kernels {
     SmallKernel sort, density, force;
-    uint32_t force_smem;
+    uint32_t force_smem, lanes;
 };
 
-template <int SYS, bool TRIM>
+template <int SYS, bool TRIM, int L>
 Kernels kernels_for()
 {
-    return {k_small_sort<SYS>, k_small_density<SYS, TRIM>, k_small_force<SYS, TRIM>,
-            (uint32_t)((kLoopThreads / 32) * (Slot<SYS>::count + 1) * kLanes * slot_stride(Slot<SYS>::words) * sizeof(float))};
+    return {k_small_sort<SYS>, k_small_density<SYS, TRIM, L>, k_small_force<SYS, TRIM, L>,
+            (uint32_t)((kLoopThreads / 32) * (Slot<SYS>::count + 1) * L * slot_stride<L>(Slot<SYS>::words) * sizeof(float)),
+            (uint32_t)L};
+}
+
+template <int L>
+Kernels kernels_of_lanes(const DevParams &p)
+{
+    if (p.system == CMAG_DAMBREAK)
+        return p.trim ? kernels_for<CMAG_DAMBREAK, true, L>() : kernels_for<CMAG_DAMBREAK, false, L>();
+    return p.system == CMAG_POISEUILLE ? kernels_for<CMAG_POISEUILLE, true, L>()
+                                       : kernels_for<CMAG_PERISTALSIS, true, L>();
 }
 
 Kernels kernels_of(const DevParams &p)
 {
-    if (p.system == CMAG_DAMBREAK) return p.trim ? kernels_for<CMAG_DAMBREAK, true>() : kernels_for<CMAG_DAMBREAK, false>();
-    return p.system == CMAG_POISEUILLE ? kernels_for<CMAG_POISEUILLE, true>() : kernels_for<CMAG_PERISTALSIS, true>();
+    return p.n <= kWideParticles ? kernels_of_lanes<8>(p) : kernels_of_lanes<4>(p);
 }
 
 cudaLaunchConfig_t sort_config(const DevParams &p, uint32_t cluster, cudaStream_t st, cudaLaunchAttribute (&attr)[2])
@@ -682,7 +701,7 @@ cudaError_t launch_small_step(const DevParams &p, const SmallStep &a, uint32_t c
     cudaError_t e = cudaLaunchKernelEx(&cfg, k.sort, p, a);
     cfg.attrs = attr + 1;  // programmatic dependent launch, no cluster
     cfg.numAttrs = 1;
-    cfg.gridDim = (uint32_t)(((uint64_t)p.n * kLanes + kLoopThreads - 1) / kLoopThreads);
+    cfg.gridDim = (uint32_t)(((uint64_t)p.n * k.lanes + kLoopThreads - 1) / kLoopThreads);
     cfg.blockDim = kLoopThreads;
     if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, k.density, p, a);
     cfg.dynamicSmemBytes = k.force_smem;

@@ -76,6 +76,10 @@ SCENES = {
     "dambreak 64 gate": lambda: dambreak(64, gate=False),
     "dambreak 64 cut": lambda: dambreak(64, cut=True),
     "dambreak 64 crowded": lambda: crowded(dambreak(64)),
+    "dambreak 74": lambda: dambreak(74),   # 11,542 particles, and
+    "dambreak 76": lambda: dambreak(76),   # 12,158: either side of 8 and 4 lanes
+    "dambreak 86 cut": lambda: dambreak(86, cut=True),
+    "dambreak 86 crowded": lambda: crowded(dambreak(86)),
     "dambreak 92": lambda: dambreak(92),   # 17,662 particles: of the largest
     "dambreak 94": lambda: dambreak(94),   # 18,422: staged
     "poiseuille 7x1": lambda: poiseuille(7, 1),
