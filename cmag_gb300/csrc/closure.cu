@@ -442,19 +442,18 @@ __global__ void __launch_bounds__(128)
 
 // ---- training: forward and backward on the tensor cores ----------------------------
 // A block of 8 warps takes tiles of 64 samples; two warps share 16 samples, each with
-// half of a layer's columns.  The forward pass is k_mlp's; each layer's slope of the
-// activation stays in registers, its BF16 activations go to shared memory.  The backward
-// products need FP32 deltas against BF16 weights or activations: a delta is split into
-// three BF16 parts (8 + 8 + 8 bits hold its 24) whose products accumulate in FP32,
-// smallest part first, so nothing is rounded that the FP32 form did not round.  Weight
-// gradients (16 rows and half the columns of each matrix to a warp) accumulate in
-// registers over all of the block's tiles and are added to global memory once.
-// 65,536 samples: 59 us (2.2 M m16n8k16 products); 66 us with one warp to 16 samples (4
-// warps of 255 registers), and 423 us in the form before, 128 samples a block on the
-// FP32 pipes with one 190 KB block an SM.  The error against 64 bits is the same (a few
-// 1e-6: activations that round the other way).  Bound by the chain of layers, five
-// block-wide barriers a tile, at four warps a scheduler, and by the last of four rounds
-// of tiles (1024 over 304 blocks).
+// half of a layer's columns.  The forward pass runs on the FP32 pipes in a fixed order
+// (forward_layer); each layer's slope of the activation stays in registers, its BF16
+// activations go to shared memory.  The backward products run on the tensor cores: they
+// need FP32 deltas against BF16 weights or activations, so a delta is split into three
+// BF16 parts (8 + 8 + 8 bits hold its 24) whose products accumulate in FP32, smallest
+// part first, and nothing is rounded that the FP32 form did not round.  Weight gradients
+// (16 rows and half the columns of each matrix to a warp) accumulate in registers over
+// all of the block's tiles and are added to global memory once.
+// 65,536 samples: 91 us; 423 us in the form before, 128 samples a block on the FP32 pipes
+// with one 190 KB block an SM (59 us with the forward pass on the tensor cores too, whose
+// activations round the other way now and then: not kept).  Bound by the forward pass's
+// instructions and the chain of layers, at four warps a scheduler.
 constexpr int kTile = 64;        // samples of a block's tile
 constexpr int kBackThreads = 256;  // two warps to 16 samples, 32 of 64 columns each
 constexpr int kXStride = 24;     // BF16 per row of inputs and output deltas (conflict-free)
@@ -521,7 +520,7 @@ __device__ __forceinline__ void activate(float (&c)[NT][4], __nv_bfloat16 *h, in
         float a[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const float z = c[nt][k], s = __fdividef(1.0f, 1.0f + expf(-z));
+            const float z = c[nt][k], s = sigmoid(z);
             a[k] = z * s;
             c[nt][k] = s * (1.0f + z * (1.0f - s));
         }
@@ -530,27 +529,36 @@ __device__ __forceinline__ void activate(float (&c)[NT][4], __nv_bfloat16 *h, in
     }
 }
 
-// c = b + h W^T for the warp's 16 rows (h in shared memory; W, b: its first output).
-template <int NT>
+// c = b + h W^T for the warp's 16 rows and 32 outputs (h in shared memory, K inputs a row;
+// W, b: the first output), each sum in FP32 from its bias over ascending inputs: the order
+// fixes every pre-activation's bits, and with them which activations round up to the next
+// BF16 value.  (On the tensor cores, whose sums round otherwise, about one activation in
+// 10,000 went the other way; a gradient moved by up to 4e-5 of itself.)
+template <int K, int WSTRIDE, int HSTRIDE>
 __device__ __forceinline__ void forward_layer(const __nv_bfloat16 *W, const float *b, const __nv_bfloat16 *h,
-                                              float (&c)[NT][4], int lane)
+                                              float (&c)[4][4], int g, int t)
 {
-    const int t = lane & 3, r = lane & 7, q = lane >> 3;
-    uint32_t a[4][4];
+    float2 s0[4], s1[4];  // rows g and g + 8, outputs nt * 8 + 2 t and the next
 #pragma unroll
-    for (int kt = 0; kt < 4; ++kt)
-        load_matrices(a[kt], h + (r + (q & 1) * 8) * kHStride + kt * 16 + (q >> 1) * 8);
+    for (int nt = 0; nt < 4; ++nt) s0[nt] = s1[nt] = make_float2(b[nt * 8 + 2 * t], b[nt * 8 + 2 * t + 1]);
+#pragma unroll 4
+    for (int k = 0; k < K; k += 2) {
+        const float2 h0 = unpack2(lds32(h + g * HSTRIDE + k)), h1 = unpack2(lds32(h + (g + 8) * HSTRIDE + k));
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-        c[nt][0] = c[nt][2] = b[nt * 8 + 2 * t];
-        c[nt][1] = c[nt][3] = b[nt * 8 + 2 * t + 1];
-#pragma unroll
-        for (int kt = 0; kt < 4; kt += 2) {
-            uint32_t w[4];
-            load_matrices(w, W + (nt * 8 + r) * kWStride + kt * 16 + q * 8);
-            mma16816(c[nt], a[kt], w[0], w[1]);
-            mma16816(c[nt], a[kt + 1], w[2], w[3]);
+        for (int nt = 0; nt < 4; ++nt) {
+            const __nv_bfloat16 *row = W + (nt * 8 + 2 * t) * WSTRIDE + k;
+            const float2 w0 = unpack2(lds32(row)), w1 = unpack2(lds32(row + WSTRIDE));
+            const float2 a = make_float2(w0.x, w1.x), e = make_float2(w0.y, w1.y);
+            s0[nt] = __ffma2_rn(e, make_float2(h0.y, h0.y), __ffma2_rn(a, make_float2(h0.x, h0.x), s0[nt]));
+            s1[nt] = __ffma2_rn(e, make_float2(h1.y, h1.y), __ffma2_rn(a, make_float2(h1.x, h1.x), s1[nt]));
         }
+    }
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+        c[nt][0] = s0[nt].x;
+        c[nt][1] = s0[nt].y;
+        c[nt][2] = s1[nt].x;
+        c[nt][3] = s1[nt].y;
     }
 }
 
@@ -673,30 +681,28 @@ __global__ void __launch_bounds__(kBackThreads, 2)
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const uint32_t r0 = tile * kTile + w0 + g, r1 = r0 + 8;
         // inputs
-        uint32_t x[1][4];
+        if (left) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int k = 2 * t + 8 * half;
-            const float m0 = cv.mean[k], m1 = cv.mean[k + 1], i0 = cv.inv_std[k], i1 = cv.inv_std[k + 1];
-            float2 f0 = make_float2(0.0f, 0.0f), f1 = f0;
-            if (r0 < n) f0 = __ldg(reinterpret_cast<const float2 *>(feat + (size_t)r0 * kFeat + k));
-            if (r1 < n) f1 = __ldg(reinterpret_cast<const float2 *>(feat + (size_t)r1 * kFeat + k));
-            x[0][2 * half] = pack2((f0.x - m0) * i0, (f0.y - m1) * i1);
-            x[0][2 * half + 1] = pack2((f1.x - m0) * i0, (f1.y - m1) * i1);
-            if (left) {
-                *reinterpret_cast<uint32_t *>(X + (w0 + g) * kXStride + k) = x[0][2 * half];
-                *reinterpret_cast<uint32_t *>(X + (w0 + g + 8) * kXStride + k) = x[0][2 * half + 1];
+            for (int half = 0; half < 2; ++half) {
+                const int k = 2 * t + 8 * half;
+                const float m0 = cv.mean[k], m1 = cv.mean[k + 1], i0 = cv.inv_std[k], i1 = cv.inv_std[k + 1];
+                float2 f0 = make_float2(0.0f, 0.0f), f1 = f0;
+                if (r0 < n) f0 = __ldg(reinterpret_cast<const float2 *>(feat + (size_t)r0 * kFeat + k));
+                if (r1 < n) f1 = __ldg(reinterpret_cast<const float2 *>(feat + (size_t)r1 * kFeat + k));
+                *reinterpret_cast<uint32_t *>(X + (w0 + g) * kXStride + k) = pack2((f0.x - m0) * i0, (f0.y - m1) * i1);
+                *reinterpret_cast<uint32_t *>(X + (w0 + g + 8) * kXStride + k) = pack2((f1.x - m0) * i0, (f1.y - m1) * i1);
             }
         }
+        pair_sync();
         // forward
         float s1[4][4], s2[4][4], c[4][4];
-        hidden_layer<1>(sw + kSW1 + n0 * kW1Stride, kW1Stride, sb + kSB1 + n0, x, s1, g, t);
+        forward_layer<kFeat, kW1Stride, kXStride>(sw + kSW1 + n0 * kW1Stride, sb + kSB1 + n0, X + w0 * kXStride, s1, g, t);
         activate(s1, H1 + w0 * kHStride + n0, g, t);
         pair_sync();
-        forward_layer(sw + kSW2 + n0 * kWStride, sb + kSB2 + n0, H1 + w0 * kHStride, s2, lane);
+        forward_layer<kHidden, kWStride, kHStride>(sw + kSW2 + n0 * kWStride, sb + kSB2 + n0, H1 + w0 * kHStride, s2, g, t);
         activate(s2, H2 + w0 * kHStride + n0, g, t);
         pair_sync();
-        forward_layer(sw + kSW3 + n0 * kWStride, sb + kSB3 + n0, H2 + w0 * kHStride, c, lane);
+        forward_layer<kHidden, kWStride, kHStride>(sw + kSW3 + n0 * kWStride, sb + kSB3 + n0, H2 + w0 * kHStride, c, g, t);
         activate(c, H3 + w0 * kHStride + n0, g, t);
         pair_sync();
         // outputs, in FP32 (three columns: a lane's 16 activations of each row, then the
