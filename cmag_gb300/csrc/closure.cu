@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(128)
 // part first, and nothing is rounded that the FP32 form did not round.  Weight gradients
 // (16 rows and half the columns of each matrix to a warp) accumulate in registers over
 // all of the block's tiles and are added to global memory once.
-// 65,536 samples: 91 us; 423 us in the form before, 128 samples a block on the FP32 pipes
+// 65,536 samples: 87 us; 423 us in the form before, 128 samples a block on the FP32 pipes
 // with one 190 KB block an SM (59 us with the forward pass on the tensor cores too, whose
 // activations round the other way now and then: not kept).  Bound by the forward pass's
 // instructions and the chain of layers, at four warps a scheduler.
@@ -541,16 +541,28 @@ __device__ __forceinline__ void forward_layer(const __nv_bfloat16 *W, const floa
     float2 s0[4], s1[4];  // rows g and g + 8, outputs nt * 8 + 2 t and the next
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) s0[nt] = s1[nt] = make_float2(b[nt * 8 + 2 * t], b[nt * 8 + 2 * t + 1]);
-#pragma unroll 4
-    for (int k = 0; k < K; k += 2) {
-        const float2 h0 = unpack2(lds32(h + g * HSTRIDE + k)), h1 = unpack2(lds32(h + (g + 8) * HSTRIDE + k));
+    auto four = [](const __nv_bfloat16 *p, float (&v)[4]) {
+        const uint2 u = *reinterpret_cast<const uint2 *>(p);
+        const float2 a = unpack2(u.x), e = unpack2(u.y);
+        v[0] = a.x, v[1] = a.y, v[2] = e.x, v[3] = e.y;
+    };
+#pragma unroll 2
+    for (int k = 0; k < K; k += 4) {
+        float h0[4], h1[4];
+        four(h + g * HSTRIDE + k, h0);
+        four(h + (g + 8) * HSTRIDE + k, h1);
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
             const __nv_bfloat16 *row = W + (nt * 8 + 2 * t) * WSTRIDE + k;
-            const float2 w0 = unpack2(lds32(row)), w1 = unpack2(lds32(row + WSTRIDE));
-            const float2 a = make_float2(w0.x, w1.x), e = make_float2(w0.y, w1.y);
-            s0[nt] = __ffma2_rn(e, make_float2(h0.y, h0.y), __ffma2_rn(a, make_float2(h0.x, h0.x), s0[nt]));
-            s1[nt] = __ffma2_rn(e, make_float2(h1.y, h1.y), __ffma2_rn(a, make_float2(h1.x, h1.x), s1[nt]));
+            float w0[4], w1[4];
+            four(row, w0);
+            four(row + WSTRIDE, w1);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float2 w = make_float2(w0[q], w1[q]);
+                s0[nt] = __ffma2_rn(w, make_float2(h0[q], h0[q]), s0[nt]);
+                s1[nt] = __ffma2_rn(w, make_float2(h1[q], h1[q]), s1[nt]);
+            }
         }
     }
 #pragma unroll
