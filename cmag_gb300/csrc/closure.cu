@@ -25,7 +25,8 @@
 // against outputs far outside the training data; none by default).  BF16
 // parameters and activations, FP32 dot products
 // on the tensor cores (the products of two BF16 values are exact in FP32).
-// Training: the loss 0.5/n sum |y - t|^2, gradients through the same forward
+// Training: the loss 0.5/n sum |y - t|^2, gradients through the same forward (its dot
+// products on the FP32 pipes)
 // (rounding treated as identity), Adam on an FP32 master copy.
 #include <cmath>
 #include <cstring>
