@@ -447,11 +447,15 @@ __global__ void __launch_bounds__(128)
 // (forward_layer); each layer's slope of the activation stays in registers, its BF16
 // activations go to shared memory.  The backward products run on the tensor cores: they
 // need FP32 deltas against BF16 weights or activations, so a delta is split into three
-// BF16 parts (8 + 8 + 8 bits hold its 24) whose products accumulate in FP32, smallest
-// part first, and nothing is rounded that the FP32 form did not round.  Weight gradients
-// (16 rows and half the columns of each matrix to a warp) accumulate in registers over
-// all of the block's tiles and are added to global memory once.
-// 65,536 samples: 87 us; 423 us in the form before, 128 samples a block on the FP32 pipes
+// BF16 parts (8 + 8 + 8 bits hold its 24), whose products are exact; their sums round
+// as FP32 ones do (mma_add).  Weight gradients (16 rows and half the columns of each
+// matrix to a warp) accumulate in registers over all of the block's tiles and are added
+// to global memory once.  Error against 64 bits on the same activations (norm of W1's
+// gradient, median of 12 seeds; FP32 pipes before / here): 64 rows 2.8e-7 / 1.7e-7,
+// 2048 2.1e-7 / 1.3e-7, 5003 1.8e-7 / 1.2e-7, 65,536 3.4e-7 / 1.1e-7; with the sums in
+// one chain on the tensor cores and one copy of the gradient 2.9e-7, -, 2.8e-7, 3.4e-7,
+// most of it a gradient shrunk by 2.3e-7 of itself.
+// 65,536 samples: 88 us; 423 us in the form before, 128 samples a block on the FP32 pipes
 // with one 190 KB block an SM (59 us with the forward pass on the tensor cores too, whose
 // activations round the other way now and then: not kept).  Bound by the forward pass's
 // instructions and the chain of layers, at four warps a scheduler.
@@ -575,60 +579,97 @@ __device__ __forceinline__ void forward_layer(const __nv_bfloat16 *W, const floa
     }
 }
 
+// d = A B: sums of 16 products from zero.
+__device__ __forceinline__ void mma16816_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+{
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+        "{%8,%9}, {%10,%10,%10,%10};\n"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+}
+
+// c += A B, MAIN: for the main part of a delta.  The tensor cores truncate a running sum
+// at every addition, always towards zero; over a chain of products that shrinks the sum
+// by up to 1e-7 of it.  So the main part's products are summed from zero, 16 at a time
+// (their 16 bits each mostly fit), and added here in FP32, rounded to nearest.  The small
+// parts (2^-8 and 2^-16 of the main one) lose nothing that counts in a chain.
+template <bool MAIN>
+__device__ __forceinline__ void mma_add(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+{
+    if (!MAIN) {
+        mma16816(c, a, b0, b1);
+        return;
+    }
+    float m[4];
+    mma16816_zero(m, a, b0, b1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] += m[i];
+}
+
 // c = d W for the warp's 16 rows (W: its first column): the deltas of the layer below
-// before its slopes.
+// before its slopes; the small parts first.
+template <bool MAIN, int NT>
+__device__ __forceinline__ void backward_part(const __nv_bfloat16 *W, const __nv_bfloat16 *d, float (&c)[NT][4],
+                                              int lane)
+{
+    const int r = lane & 7, q = lane >> 3;
+#pragma unroll
+    for (int kt = 0; kt < 4; ++kt) {
+        uint32_t a[4];
+        load_matrices(a, d + (r + (q & 1) * 8) * kHStride + kt * 16 + (q >> 1) * 8);
+#pragma unroll
+        for (int nt = 0; nt < NT; nt += 2) {
+            uint32_t w[4];
+            load_matrices_trans(w, W + (kt * 16 + (q & 1) * 8 + r) * kWStride + nt * 8 + (q >> 1) * 8);
+            mma_add<MAIN>(c[nt], a, w[0], w[1]);
+            mma_add<MAIN>(c[nt + 1], a, w[2], w[3]);
+        }
+    }
+}
 template <int NT>
 __device__ __forceinline__ void backward_layer(const __nv_bfloat16 *W, const __nv_bfloat16 *d, float (&c)[NT][4],
                                                int lane)
 {
-    const int r = lane & 7, q = lane >> 3;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.0f;
 #pragma unroll 1
-    for (int part = 2; part >= 0; --part) {
-#pragma unroll
-        for (int kt = 0; kt < 4; ++kt) {
-            uint32_t a[4];
-            load_matrices(a, d + part * kPlane + (r + (q & 1) * 8) * kHStride + kt * 16 + (q >> 1) * 8);
-#pragma unroll
-            for (int nt = 0; nt < NT; nt += 2) {
-                uint32_t w[4];
-                load_matrices_trans(w, W + (kt * 16 + (q & 1) * 8 + r) * kWStride + nt * 8 + (q >> 1) * 8);
-                mma16816(c[nt], a, w[0], w[1]);
-                mma16816(c[nt + 1], a, w[2], w[3]);
-            }
-        }
-    }
+    for (int part = 2; part >= 1; --part) backward_part<false>(W, d + part * kPlane, c, lane);
+    backward_part<true>(W, d, c, lane);
 }
 
 // g[nt] += sum over the tile's samples of d[s][m0 ..] h[s][nt * 8 ..], and the same
-// against ones into gb (bias: in one warp of those that share m0).  The tile's products are summed from zero, the small parts
-// first, and then added: the tensor cores' additions lose up to a unit in the last
-// place of the sum each, always towards zero, which over many tiles shrank the
-// gradient by 8e-7 of it.
+// against ones into gb (bias: in one warp of those that share m0).  A tile's products are
+// summed from zero, the small parts first, and then added.
+template <bool MAIN, int NT, int DSTRIDE, int HSTRIDE>
+__device__ __forceinline__ void grad_part(float (&a0)[NT][4], float (&ab)[4], const __nv_bfloat16 *d, int m0,
+                                          const __nv_bfloat16 *h, bool bias, int lane)
+{
+    constexpr uint32_t kOnes = 0x3f803f80u;
+    const int r = lane & 7, q = lane >> 3;
+#pragma unroll
+    for (int s0 = 0; s0 < kTile; s0 += 16) {
+        uint32_t a[4];
+        load_matrices_trans(a, d + (s0 + (q >> 1) * 8 + r) * DSTRIDE + m0 + (q & 1) * 8);
+#pragma unroll
+        for (int k = 0; k < NT / 2; ++k) {
+            uint32_t b[4];
+            load_matrices_trans(b, h + (s0 + (q & 1) * 8 + r) * HSTRIDE + k * 16 + (q >> 1) * 8);
+            mma_add<MAIN>(a0[2 * k], a, b[0], b[1]);
+            mma_add<MAIN>(a0[2 * k + 1], a, b[2], b[3]);
+        }
+        if (bias) mma_add<MAIN>(ab, a, kOnes, kOnes);
+    }
+}
 template <int NT, int DSTRIDE, int HSTRIDE>
 __device__ __forceinline__ void weight_grad(float (&g)[NT][4], float (&gb)[4], const __nv_bfloat16 *d, int plane,
                                             int m0, const __nv_bfloat16 *h, bool bias, int lane)
 {
-    constexpr uint32_t kOnes = 0x3f803f80u;
-    const int r = lane & 7, q = lane >> 3;
     float a0[NT][4] = {}, ab[4] = {};
 #pragma unroll 1
-    for (int part = 2; part >= 0; --part) {
-#pragma unroll
-        for (int s0 = 0; s0 < kTile; s0 += 16) {
-            uint32_t a[4];
-            load_matrices_trans(a, d + part * plane + (s0 + (q >> 1) * 8 + r) * DSTRIDE + m0 + (q & 1) * 8);
-#pragma unroll
-            for (int k = 0; k < NT / 2; ++k) {
-                uint32_t b[4];
-                load_matrices_trans(b, h + (s0 + (q & 1) * 8 + r) * HSTRIDE + k * 16 + (q >> 1) * 8);
-                mma16816(a0[2 * k], a, b[0], b[1]);
-                mma16816(a0[2 * k + 1], a, b[2], b[3]);
-            }
-            if (bias) mma16816(ab, a, kOnes, kOnes);
-        }
-    }
+    for (int part = 2; part >= 1; --part)
+        grad_part<false, NT, DSTRIDE, HSTRIDE>(a0, ab, d + part * plane, m0, h, bias, lane);
+    grad_part<true, NT, DSTRIDE, HSTRIDE>(a0, ab, d, m0, h, bias, lane);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         gb[i] += ab[i];
@@ -664,7 +705,8 @@ __device__ __forceinline__ void multiply_store(float (&c)[4][4], const float (&s
     }
 }
 
-// Loss and gradient over n samples; both are added to global FP32 accumulators.
+// Loss and gradient over n samples; both are added to global FP32 accumulators, the
+// gradient to one of kGradCopies of them (closure.h).
 __global__ void __launch_bounds__(kBackThreads, 2)
     k_backward(ClosureView cv, const float *__restrict__ feat, const float *__restrict__ target, uint32_t n,
                float *__restrict__ grad, float *__restrict__ loss)
@@ -780,6 +822,7 @@ __global__ void __launch_bounds__(kBackThreads, 2)
         if (left) weight_grad<2, kHStride, kXStride>(ge, gbe, D, kPlane, w0, X, true, lane);
         __syncthreads();
     }
+    grad += (blockIdx.x % kGradCopies) * kGradStride;
     add_gradient(grad + kOffW2, kHidden, g2, w0 + g, kHidden, n0, t);
     add_gradient(grad + kOffW3, kHidden, g3, w0 + g, kHidden, n0, t);
     if (left) add_gradient(grad + kOffW1, kFeat, ge, w0 + g, kHidden, 0, t);
@@ -822,12 +865,28 @@ __device__ __forceinline__ void update_image(uint32_t *image, int k, float v)
     else reinterpret_cast<__nv_bfloat16 *>(image)[base + row * stride + col] = __float2bfloat16_rn(v);
 }
 
+// The gradient of parameter k: the sum of its copies.
+__device__ __forceinline__ float gradient_of(const float *grad, int k)
+{
+    double g = 0.0;
+#pragma unroll
+    for (int c = 0; c < kGradCopies; ++c) g += (double)grad[c * kGradStride + k];
+    return (float)g;
+}
+
+// Leaves the gradient in its first copy.
+__global__ void k_fold_gradient(float *grad)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < kClosureParams) grad[k] = gradient_of(grad, k);
+}
+
 __global__ void k_adam(float *master, float *m, float *v, float *grad, __nv_bfloat16 *w, uint32_t *image,
                        float lr, float beta1, float beta2, float eps, float bias1, float bias2)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= kClosureParams) return;
-    const float g = grad[k];
+    const float g = gradient_of(grad, k);
     const float mk = beta1 * m[k] + (1.0f - beta1) * g;
     const float vk = beta2 * v[k] + (1.0f - beta2) * g * g;
     m[k] = mk;
@@ -837,7 +896,8 @@ __global__ void k_adam(float *master, float *m, float *v, float *grad, __nv_bflo
     master[k] = nw;
     w[k] = __float2bfloat16_rn(nw);
     update_image(image, k, nw);
-    grad[k] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < kGradCopies; ++c) grad[c * kGradStride + k] = 0.0f;
 }
 
 __global__ void k_round(const float *master, __nv_bfloat16 *w)
@@ -981,6 +1041,11 @@ void launch_closure_backward(const ClosureView &c, const float *feat, const floa
     allow_smem(k_backward, kSmemBackward);
     const uint32_t tiles = (n + kTile - 1) / kTile, most = 2u * (uint32_t)device_sm_count();  // 2 blocks an SM
     k_backward<<<tiles < most ? tiles : most, kBackThreads, kSmemBackward, st>>>(c, feat, target, n, grad, loss);
+}
+
+void launch_closure_fold(float *grad, cudaStream_t st)
+{
+    k_fold_gradient<<<(kClosureParams + 255) / 256, 256, 0, st>>>(grad);
 }
 
 uint32_t closure_image_words() { return (uint32_t)kImageWords; }

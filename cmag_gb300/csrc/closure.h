@@ -62,10 +62,17 @@ void launch_interpolate(const DevParams &p, const float4 *spos, const float2 *au
 // Network outputs (unscaled) for n raw feature rows (xb: n x 16 BF16 scratch).
 void launch_closure_forward(const ClosureView &c, const float *feat, uint32_t n,
                             __nv_bfloat16 *xb, float *out, cudaStream_t st);
+// The blocks of a backward pass add their gradients to kGradCopies FP32 copies in turn,
+// so that a chain of rounded additions is a quarter as long; the copies are summed in
+// 64 bits where the gradient is used.  kGradStride floats apart (8-byte aligned).
+constexpr int kGradCopies = 4;
+constexpr int kGradStride = (kClosureParams + 1) & ~1;
 // Loss 0.5/n sum |y - t|^2 over n rows (t: targets, n x 3) added to *loss and its
-// gradient with respect to the BF16 parameters added to grad (FP32).
+// gradient with respect to the BF16 parameters added to the copies in grad (FP32).
 void launch_closure_backward(const ClosureView &c, const float *feat, const float *target,
                              uint32_t n, float *grad, float *loss, cudaStream_t st);
+// Sums the copies into the first one (kClosureParams values).
+void launch_closure_fold(float *grad, cudaStream_t st);
 // Adam on the FP32 master copy; refreshes the BF16 copy and its shared-memory
 // image and clears grad.
 void launch_closure_adam(float *master, float *m, float *v, float *grad, __nv_bfloat16 *w,
@@ -78,7 +85,8 @@ void launch_closure_round(const float *master, __nv_bfloat16 *w, uint4 *image, c
 
 // A trainable network instance (C ABI handle).
 struct cmag_closure {
-    float *master = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr;  // FP32, kClosureParams
+    float *master = nullptr, *m = nullptr, *v = nullptr;                   // FP32, kClosureParams
+    float *grad = nullptr;                                                 // kGradCopies x kGradStride
     __nv_bfloat16 *w = nullptr;                                            // BF16 copy used by kernels
     uint4 *image = nullptr;                                                // w as the network kernel stages it
     float *norm = nullptr;   // mean[16], inv_std[16], out_scale, loss, out_limit

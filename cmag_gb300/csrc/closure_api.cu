@@ -42,6 +42,7 @@ void free_all(cmag_closure *c)
     if (c->stream) cudaStreamDestroy(c->stream);
 }
 
+constexpr size_t kGradBytes = sizeof(float) * kGradCopies * kGradStride;
 constexpr size_t kNormFloats = 2 * kFeat + 3;  // mean, inv_std, out_scale, loss, out_limit
 
 }  // namespace
@@ -61,13 +62,13 @@ int cmag_closure_create(const float *params, cmag_closure **out)
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->master, pb);
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->m, pb);
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->v, pb);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&c->grad, pb);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&c->grad, kGradBytes);
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->w, sizeof(__nv_bfloat16) * kClosureParams);
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->norm, sizeof(float) * kNormFloats);
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->image, sizeof(uint4) * closure_image_words());
     if (e == cudaSuccess) e = cudaMemset(c->m, 0, pb);
     if (e == cudaSuccess) e = cudaMemset(c->v, 0, pb);
-    if (e == cudaSuccess) e = cudaMemset(c->grad, 0, pb);
+    if (e == cudaSuccess) e = cudaMemset(c->grad, 0, kGradBytes);
     if (e == cudaSuccess) {
         std::vector<float> init(kClosureParams, 0.0f), norm(kNormFloats, 0.0f);
         if (params) std::memcpy(init.data(), params, pb);
@@ -200,15 +201,16 @@ int cmag_closure_gradient(cmag_closure *c, const float *d_features, const float 
     if (!c || !grad_out || (n && (!d_features || !d_targets)))
         return cfail(c, CMAG_ERR_INVALID, "null argument");
     cudaStream_t st = stream_of(c, stream);
-    CC_CUDA(c, cudaMemsetAsync(c->grad, 0, sizeof(float) * kClosureParams, st));
+    CC_CUDA(c, cudaMemsetAsync(c->grad, 0, kGradBytes, st));
     CC_CUDA(c, cudaMemsetAsync(c->loss(), 0, sizeof(float), st));
     launch_closure_backward(c->view(), d_features, d_targets, n, c->grad, c->loss(), st);
+    launch_closure_fold(c->grad, st);
     CC_CUDA(c, cudaGetLastError());
     CC_CUDA(c, cudaMemcpyAsync(grad_out, c->grad, sizeof(float) * kClosureParams,
                                cudaMemcpyDeviceToHost, st));
     float l = 0.0f;
     CC_CUDA(c, cudaMemcpyAsync(&l, c->loss(), sizeof(float), cudaMemcpyDeviceToHost, st));
-    CC_CUDA(c, cudaMemsetAsync(c->grad, 0, sizeof(float) * kClosureParams, st));
+    CC_CUDA(c, cudaMemsetAsync(c->grad, 0, kGradBytes, st));
     CC_CUDA(c, cudaStreamSynchronize(st));
     if (loss_out) *loss_out = l;
     return CMAG_OK;
@@ -241,7 +243,7 @@ int cmag_closure_reset_optimizer(cmag_closure *c)
     c->adam_steps = 0;
     CC_CUDA(c, cudaMemsetAsync(c->m, 0, sizeof(float) * kClosureParams, c->stream));
     CC_CUDA(c, cudaMemsetAsync(c->v, 0, sizeof(float) * kClosureParams, c->stream));
-    CC_CUDA(c, cudaMemsetAsync(c->grad, 0, sizeof(float) * kClosureParams, c->stream));
+    CC_CUDA(c, cudaMemsetAsync(c->grad, 0, kGradBytes, c->stream));
     CC_CUDA(c, cudaStreamSynchronize(c->stream));
     return CMAG_OK;
 }
