@@ -741,7 +741,13 @@ bool small_steps(cmag_system *s) { return s->g_density == 1 && s->g_force == 1 &
 
 int do_step(cmag_system *s)
 {
-    if (small_steps(s)) {
+    bool small = small_steps(s);
+    if (small) {  // on a stream that its owner captures a step is refused, as the staged one's graph is
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        CM_CUDA(s, cudaStreamIsCapturing(st_of(s), &capture));
+        small = capture == cudaStreamCaptureStatusNone;
+    }
+    if (small) {
         const bool per = s->p.system == CMAG_PERISTALSIS;
         const SmallStep a{s->pos, s->vel, s->vlf, s->meas, s->spos, s->svel, per ? s->vforce : s->acc,
                           per ? s->pforce : nullptr, s->aux, s->hash[0], s->idx[0], s->hash[1], s->idx[1],
