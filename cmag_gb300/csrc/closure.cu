@@ -43,6 +43,7 @@ namespace {
 
 constexpr int kWalkThreads = 128;  // per block of the feature and interpolation walks
 constexpr int kInterpLanes = 4;    // lanes that share an interpolation point
+constexpr uint32_t kInterpPoints = kWalkThreads / kInterpLanes;  // points of a block
 
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
@@ -920,7 +921,8 @@ __global__ void __launch_bounds__(kWalkThreads)
              float4 *__restrict__ out)
 {
     pdl_entry();
-    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / kInterpLanes;
+    // (from the block's points: four threads a point pass 2^32 at 2^30 points)
+    const uint32_t t = blockIdx.x * kInterpPoints + threadIdx.x / kInterpLanes;
     const float4 q = pts[min(t, n - 1)];
     float sx = 0.f, sy = 0.f, sz = 0.f, sw = 0.f;
     for_each_two<PLANAR, TRIM, kInterpLanes>(p, spos, off, threadIdx.x % kInterpLanes, q, [&](uint32_t j, const float4 &a, const float4 &b, bool two) {
@@ -1021,8 +1023,7 @@ void launch_interpolate(const DevParams &p, const float4 *spos, const float2 *au
 {
     if (n == 0) return;
     launch_pdl(k_neighbor_values<true>, (p.n + 255) / 256, 256, 0, st, p.mass, arr, aux, idx, p.n, nval);
-    constexpr uint32_t kPoints = kWalkThreads / kInterpLanes;  // of a block
-    const uint32_t blocks = (n + kPoints - 1) / kPoints;
+    const uint32_t blocks = (n - 1) / kInterpPoints + 1;
 #define CMAG_INTERP(PL, TR) launch_pdl(k_interp<PL, TR>, blocks, kWalkThreads, 0, st, p, spos, nval, off, pts, n, out)
     if (p.planar) {
         if (p.trim) CMAG_INTERP(true, true);
