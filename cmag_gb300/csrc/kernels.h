@@ -195,6 +195,7 @@ struct SmallStep {
     uint32_t *hash, *rank, *shash, *tmp, *idx, *cnt, *off, *err;
     PhaseState *phase;
     float k_milli;
+    bool lists;  // interaction lists are on: the force takes the pairs they would hold
 };
 // Whether the scene is of this kind (single planar scenes, one lane per particle).
 bool small_step_fits(const DevParams &p);

@@ -18,6 +18,7 @@ struct PairSelf {
     float2 aux;    // p/rho^2, and rho (DamBreak) or 1/rho
     float nmass;   // -mass: pressure factor
     float visc_i;  // viscous factor of the particle
+    bool lists;    // take the pairs that interaction lists hold
 };
 
 // DamBreak: sum += a r.  Poiseuille: sum += a r, then b v.  Peristalsis: pressure
@@ -102,7 +103,9 @@ __device__ __forceinline__ bool pair_terms(const DevParams &p, const PairSelf &s
     const float d2 = pair_distance<SYS, PLANAR>(s, pj, sx, sy, sz, t);
     // (a coincident pair has no direction: it contributes nothing)
     const bool wall = SYS == CMAG_DAMBREAK && pj.w != (float)CMAG_FLUID;
-    const bool hit = j != s.i && d2 != 0.0f && (d2 < p.support2 || (wall && !TRIM));
+    // a wall without cut-off at a distance that is not a number: the walk takes it, lists
+    // do not hold it
+    const bool hit = j != s.i && d2 != 0.0f && (d2 < p.support2 || (wall && !TRIM && (!s.lists || d2 > 0.0f)));
     pair_factors<SYS, PLANAR>(p, s, pj, d2, vj, aj, t);
     if (wall) t.a = wall_factor(p, d2);
     if (!hit) t = PairTerms{};

@@ -268,6 +268,13 @@ __device__ __forceinline__ float4 pair_weights(const DevParams &p, float4 pi, fl
                : make_float4(__fmul_rn(t4.x, lin.x), 1.0f, 0.0f, 0.0f);
 }
 
+// Whether a term (w.x w.y, w.z w.w) changes a sum: a factor (1 - q/2)^4 is not zero, or the
+// other one is NaN, of a candidate that is not at a finite place (0 * NaN is NaN).
+__device__ __forceinline__ bool counts(float4 w)
+{
+    return w.x != 0.0f || w.z != 0.0f || isnan(w.y + w.w);
+}
+
 // A cubic-spline candidate's weight (density.cu).
 template <int SYS>
 __device__ __forceinline__ float spline_weight(const DevParams &p, float4 pi, float4 pj, float sx, float sy)
@@ -308,12 +315,12 @@ template <int SYS, int L>
 __device__ __forceinline__ bool add_rows(const DevParams &p, const float4 *spos, const Group<L> &gr, const Row &row,
                                          float4 pi, float *s, float &sum)
 {
-    // a term is stored behind the row's earlier ones and counted when it is not zero
+    // a term is stored behind the row's earlier ones and counted when it changes the sum
     // (no branch); the slot after the last is scratch
     uint32_t at = 0;
     auto put = [&](float4 w) {
         *reinterpret_cast<float4 *>(s + gr.slot(min(at, (uint32_t)kSlots), gr.lane, 4)) = w;
-        at += (w.x != 0.0f || w.z != 0.0f) ? 1u : 0u;
+        at += counts(w) ? 1u : 0u;
     };
     const bool wendland = p.kernel == CMAG_KERNEL_WENDLAND;
     if (wendland) {
@@ -335,7 +342,7 @@ __device__ __forceinline__ bool add_rows(const DevParams &p, const float4 *spos,
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) {
                 float4 w = pair_weights<SYS>(p, pi, q0[u], q1[u], two[u], m0 + u < h0 ? row.sx0 : row.sx1, row.sy);
-                if (m0 + u >= h) w.x = w.z = 0.0f;
+                if (m0 + u >= h) w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 put(w);
             }
         }
@@ -389,7 +396,7 @@ __device__ __noinline__ float add_long_rows(const DevParams &p, const float4 *sp
                         w = make_float4(spline_weight<SYS>(p, pi, q, sx, row.sy), 1.0f, 0.0f, 0.0f);
                     }
                 }
-                if (gr.all(w.x == 0.0f && w.z == 0.0f)) continue;  // out of reach: nothing to add
+                if (gr.all(!counts(w))) continue;  // out of reach: nothing to add
                 *reinterpret_cast<float4 *>(s + gr.slot(0, gr.lane, 4)) = w;
                 gr.sync();
                 if (gr.lane < (int)per) {
@@ -586,7 +593,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_small_force(DevParams p, Sm
     if (SYS == CMAG_DAMBREAK && pi.w != (float)CMAG_FLUID) return;
     const float4 vi = __ldg(a.svel + i);
     const float2 ai = __ldg(a.aux + i);
-    const PairSelf self{i, pi, vi, ai, -p.mass, p.visc_coeff * ai.y};
+    const PairSelf self{i, pi, vi, ai, -p.mass, p.visc_coeff * ai.y, a.lists};
     const int3 g = grid_pos(p, pi.x, pi.y, pi.z);
     const float3 f = walk::frac_cell(p, pi);
     float sum = 0.0f;

@@ -751,7 +751,7 @@ int do_step(cmag_system *s)
         const bool per = s->p.system == CMAG_PERISTALSIS;
         const SmallStep a{s->pos, s->vel, s->vlf, s->meas, s->spos, s->svel, per ? s->vforce : s->acc,
                           per ? s->pforce : nullptr, s->aux, s->hash[0], s->idx[0], s->hash[1], s->idx[1],
-                          s->idx[0], s->cnt, s->off, s->err, s->phase, s->k_milli};
+                          s->idx[0], s->cnt, s->off, s->err, s->phase, s->k_milli, s->nl_entry != nullptr};
         CM_CUDA(s, launch_small_step(s->small_dev, a, s->small_cluster, st_of(s)));
         if (s->vl_flags) verlet_force(s);
     } else if (s->use_graphs && !s->timing && s->stream != nullptr) {
