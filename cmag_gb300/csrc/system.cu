@@ -84,6 +84,9 @@ struct cmag_system {
     // scratch of the feature and interpolation walks (n): behind wc_snap, or made on first use
     float4 *nval = nullptr;
     bool nval_own = false;
+    // held while a step's launches, or a query's two, are enqueued: a query fills nval in
+    // one launch and reads it in the next, and several host threads may query one system
+    std::mutex launch_mu;
 
     bool use_graphs = true;
     cudaGraphExec_t gexec = nullptr;
@@ -741,6 +744,7 @@ bool small_steps(cmag_system *s) { return s->g_density == 1 && s->g_force == 1 &
 
 int do_step(cmag_system *s)
 {
+    std::lock_guard<std::mutex> lock(s->launch_mu);
     bool small = small_steps(s);
     if (small) {  // on a stream that its owner captures a step is refused, as the staged one's graph is
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -1331,7 +1335,11 @@ int cmag_system_run_stages(cmag_system *s, int32_t last_stage)
     if (!s) return fail(nullptr, CMAG_ERR_INVALID, "null handle");
     if (last_stage < CMAG_STAGE_HASH || last_stage > CMAG_STAGE_INTEGRATE)
         return fail(s, CMAG_ERR_INVALID, "unknown stage");
-    int rc = record_step(s, last_stage, false);
+    int rc = CMAG_OK;
+    {
+        std::lock_guard<std::mutex> lock(s->launch_mu);
+        rc = record_step(s, last_stage, false);
+    }
     if (rc != CMAG_OK) return rc;
     s->last_stage = last_stage;
     if (last_stage == CMAG_STAGE_INTEGRATE) {
@@ -1572,6 +1580,7 @@ int cmag_system_autotune(cmag_system *s, int32_t reps)
     if (!s) return fail(nullptr, CMAG_ERR_INVALID, "null handle");
     if (reps < 1) reps = 1;
     if (s->vl_skin > 0.0f) return CMAG_OK;  // kept lists: one lane per particle, nothing to choose
+    std::lock_guard<std::mutex> lock(s->launch_mu);
     // hash, sort and gather of the current state, then time each variant
     PhaseState saved = s->host_phase;
     int rc = record_step(s, CMAG_STAGE_REORDER, false);
@@ -1738,6 +1747,7 @@ int cmag_system_set_closure(cmag_system *s, cmag_closure *c)
     if (!s) return fail(nullptr, CMAG_ERR_INVALID, "null handle");
     if (c && s->p.system != CMAG_DAMBREAK)
         return fail(s, CMAG_ERR_STATE, "the learned closure corrects DamBreak scenes only");
+    std::lock_guard<std::mutex> lock(s->launch_mu);
     if (c)
         if (int rc = ensure_nval(s)) return rc;
     if (c && !s->closure_x)
@@ -1753,10 +1763,13 @@ int cmag_system_closure_features(cmag_system *s, float *d_features)
     if (s->p.system != CMAG_DAMBREAK) return fail(s, CMAG_ERR_STATE, "not a dam-break system");
     if (s->last_stage < CMAG_STAGE_FORCE)
         return fail(s, CMAG_ERR_STATE, "features need this step's density and forces (run_stages FORCE)");
-    if (int rc = ensure_nval(s)) return rc;
-    launch_closure_features(make_dev(s), s->spos, s->svel, s->aux, s->meas, sorted_idx(s), s->off,
-                            s->acc, s->nval, d_features, st_of(s));
-    CM_CUDA(s, cudaGetLastError());
+    {
+        std::lock_guard<std::mutex> lock(s->launch_mu);
+        if (int rc = ensure_nval(s)) return rc;
+        launch_closure_features(make_dev(s), s->spos, s->svel, s->aux, s->meas, sorted_idx(s), s->off,
+                                s->acc, s->nval, d_features, st_of(s));
+        CM_CUDA(s, cudaGetLastError());
+    }
     CM_CUDA(s, cudaStreamSynchronize(st_of(s)));
     return CMAG_OK;
 }
@@ -1776,11 +1789,14 @@ int cmag_system_interpolate(cmag_system *s, int32_t array, const float *d_points
     case CMAG_VELOCITYLEAPFROG: a = s->vlf; break;
     default: return fail(s, CMAG_ERR_INVALID, "not an original-order float4 array: " + std::to_string(array));
     }
-    if (int rc = ensure_nval(s)) return rc;
-    launch_interpolate(make_dev(s), s->spos, s->aux, sorted_idx(s), s->off, a, s->nval,
-                       reinterpret_cast<const float4 *>(d_points), n, reinterpret_cast<float4 *>(d_out),
-                       st_of(s));
-    CM_CUDA(s, cudaGetLastError());
+    {
+        std::lock_guard<std::mutex> lock(s->launch_mu);
+        if (int rc = ensure_nval(s)) return rc;
+        launch_interpolate(make_dev(s), s->spos, s->aux, sorted_idx(s), s->off, a, s->nval,
+                           reinterpret_cast<const float4 *>(d_points), n, reinterpret_cast<float4 *>(d_out),
+                           st_of(s));
+        CM_CUDA(s, cudaGetLastError());
+    }
     CM_CUDA(s, cudaStreamSynchronize(st_of(s)));
     return CMAG_OK;
 }

@@ -578,7 +578,9 @@ int cmag_system_closure_features(cmag_system *s, float *d_features);
  * ACCELERATION or VELOCITYLEAPFROG) over the fluid particles of a DamBreak system,
  * at n points (device, n x 4 floats; .w ignored): d_out (device, n x 4) gets
  * sum V_j W a_j / sum V_j W in xyz and sum V_j W in w (0: no fluid in reach).
- * Uses the sorted state and densities of the last run_stages (>= DENSITY). */
+ * Uses the sorted state and densities of the last run_stages (>= DENSITY).
+ * Several host threads may call this and cmag_system_closure_features on one system at
+ * the same time. */
 int cmag_system_interpolate(cmag_system *s, int32_t array, const float *d_points, uint32_t n,
                             float *d_out);
 
