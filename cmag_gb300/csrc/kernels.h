@@ -83,8 +83,8 @@ struct SortWorkspace {
 SortWorkspace sort_workspace_view(uint32_t *base, uint32_t n);
 
 // Stable sort of n pairs on `passes` 8-bit digits; alt_*: n words of scratch each.
-void launch_sort(uint32_t *keys, uint32_t *vals, uint32_t *alt_keys, uint32_t *alt_vals, uint32_t n, int passes,
-                 const SortWorkspace &ws, uint32_t *err, cudaStream_t st);
+cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t *alt_keys, uint32_t *alt_vals, uint32_t n,
+                        int passes, const SortWorkspace &ws, uint32_t *err, cudaStream_t st);
 
 // ---- cells (cells.cu) --------------------------------------------------------
 // Hash every particle and count particles per cell.  rank (may be null): per

@@ -350,62 +350,78 @@ SortWorkspace sort_workspace_view(uint32_t *base, uint32_t n)
     return ws;
 }
 
-void launch_digit_hist(const uint32_t *keys, uint32_t n, int passes, const SortWorkspace &ws,
-                       const uint32_t *vals, uint32_t *ckeys, uint32_t *cvals, cudaStream_t st)
+namespace {
+
+// A plain launch that returns its own error (not one that the caller left pending).
+template <typename... KArgs, typename... Args>
+cudaError_t launch(void (*kernel)(KArgs...), uint32_t blocks, uint32_t threads, size_t smem, cudaStream_t st,
+                   Args... args)
 {
-    if (n == 0 || passes == 0) return;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = blocks;
+    cfg.blockDim = threads;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+cudaError_t launch_digit_hist(const uint32_t *keys, uint32_t n, int passes, const SortWorkspace &ws,
+                              const uint32_t *vals, uint32_t *ckeys, uint32_t *cvals, cudaStream_t st)
+{
     uint32_t blocks = (n + 2047) / 2048;
     const uint32_t cap = 8u * (uint32_t)device_sm_count();  // 8 blocks per SM
     if (blocks > cap) blocks = cap;
     const uint32_t status_words4 = (uint32_t)((size_t)passes * status_words(n) / 4);
-    k_digit_hist<<<blocks, 256, 0, st>>>(keys, n, passes, ws.hist, reinterpret_cast<uint4 *>(ws.status),
-                                         status_words4, vals, ckeys, cvals);
+    return launch(k_digit_hist, blocks, 256, 0, st, keys, n, passes, ws.hist, reinterpret_cast<uint4 *>(ws.status),
+                  status_words4, vals, ckeys, cvals);
 }
-
-namespace {
 
 template <int kItems>
-void launch_pass(const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout, uint32_t n, int pass,
-                 const SortWorkspace &ws, uint32_t *err, cudaStream_t st)
+cudaError_t launch_pass(const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout, uint32_t n, int pass,
+                        const SortWorkspace &ws, uint32_t *err, cudaStream_t st)
 {
     constexpr int bytes = 2 * kSortThreads * kItems * (int)sizeof(uint32_t);  // a tile's pairs
-    if (pass == 0) cudaFuncSetAttribute(k_onesweep<kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (pass == 0) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(k_onesweep<kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return e;
+    }
     const uint32_t tiles = sort_tiles(n);
     uint32_t *status = ws.status + (size_t)pass * status_words(n);
-    k_onesweep<kItems><<<tiles, kSortThreads, bytes, st>>>(kin, vin, kout, vout, n, 8 * pass, ws.hist + pass * kRadix,
-                                                           ws.tile_ctr + pass, status,
-                                                           status + (size_t)tiles * kRadix, err);
+    return launch(k_onesweep<kItems>, tiles, kSortThreads, bytes, st, kin, vin, kout, vout, n, 8 * pass,
+                  ws.hist + pass * kRadix, ws.tile_ctr + pass, status, status + (size_t)tiles * kRadix, err);
 }
 
-void launch_onesweep_pass(const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout, uint32_t n,
-                          int pass, const SortWorkspace &ws, uint32_t *err, cudaStream_t st)
+cudaError_t launch_onesweep_pass(const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout,
+                                 uint32_t n, int pass, const SortWorkspace &ws, uint32_t *err, cudaStream_t st)
 {
     switch (sort_items(n)) {
-    case 1: launch_pass<1>(kin, vin, kout, vout, n, pass, ws, err, st); break;
-    case 2: launch_pass<2>(kin, vin, kout, vout, n, pass, ws, err, st); break;
-    case 3: launch_pass<3>(kin, vin, kout, vout, n, pass, ws, err, st); break;
-    case 4: launch_pass<4>(kin, vin, kout, vout, n, pass, ws, err, st); break;
-    case 5: launch_pass<5>(kin, vin, kout, vout, n, pass, ws, err, st); break;
-    case 6: launch_pass<6>(kin, vin, kout, vout, n, pass, ws, err, st); break;
-    case 7: launch_pass<7>(kin, vin, kout, vout, n, pass, ws, err, st); break;
-    default: launch_pass<8>(kin, vin, kout, vout, n, pass, ws, err, st); break;
+    case 1: return launch_pass<1>(kin, vin, kout, vout, n, pass, ws, err, st);
+    case 2: return launch_pass<2>(kin, vin, kout, vout, n, pass, ws, err, st);
+    case 3: return launch_pass<3>(kin, vin, kout, vout, n, pass, ws, err, st);
+    case 4: return launch_pass<4>(kin, vin, kout, vout, n, pass, ws, err, st);
+    case 5: return launch_pass<5>(kin, vin, kout, vout, n, pass, ws, err, st);
+    case 6: return launch_pass<6>(kin, vin, kout, vout, n, pass, ws, err, st);
+    case 7: return launch_pass<7>(kin, vin, kout, vout, n, pass, ws, err, st);
+    default: return launch_pass<8>(kin, vin, kout, vout, n, pass, ws, err, st);
     }
 }
 
 }  // namespace
 
 // The sort of n pairs on a zeroed head of the workspace (sort_head_words() words): the
-// result is in keys / vals; alt_*: n words of scratch each.
-void launch_sort(uint32_t *keys, uint32_t *vals, uint32_t *alt_keys, uint32_t *alt_vals, uint32_t n, int passes,
-                 const SortWorkspace &ws, uint32_t *err, cudaStream_t st)
+// result is in keys / vals; alt_*: n words of scratch each.  A launch that fails ends it.
+cudaError_t launch_sort(uint32_t *keys, uint32_t *vals, uint32_t *alt_keys, uint32_t *alt_vals, uint32_t n,
+                        int passes, const SortWorkspace &ws, uint32_t *err, cudaStream_t st)
 {
     const bool odd = passes & 1;
-    launch_digit_hist(keys, n, passes, ws, vals, odd ? alt_keys : nullptr, odd ? alt_vals : nullptr, st);
+    cudaError_t e = launch_digit_hist(keys, n, passes, ws, vals, odd ? alt_keys : nullptr, odd ? alt_vals : nullptr, st);
     uint32_t *kb[2] = {keys, alt_keys}, *vb[2] = {vals, alt_vals};
-    for (int k = 0; k < passes; ++k) {
+    for (int k = 0; k < passes && e == cudaSuccess; ++k) {
         const int src = (k & 1) ^ (odd ? 1 : 0), dst = src ^ 1;
-        launch_onesweep_pass(kb[src], vb[src], kb[dst], vb[dst], n, k, ws, err, st);
+        e = launch_onesweep_pass(kb[src], vb[src], kb[dst], vb[dst], n, k, ws, err, st);
     }
+    return e;
 }
 
 }  // namespace cmag
@@ -541,10 +557,10 @@ int cmag_sort_particles_noalloc(uint32_t *d_hash, uint32_t *d_index, uint32_t n,
     cudaError_t e = cudaMemsetAsync(base, 0, sort_head_words() * sizeof(uint32_t), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return noalloc_fail(CMAG_ERR_CUDA, "cudaMemsetAsync", e);
-    launch_sort(d_hash, d_index, alt_keys, alt_vals, n, passes, sort_workspace_view(base, n), err, st);
+    e = launch_sort(d_hash, d_index, alt_keys, alt_vals, n, passes, sort_workspace_view(base, n), err, st);
     // a launch that failed leaves its error pending; it is reported but not
     // cleared (an error left by the caller's earlier work stays the caller's)
-    e = cudaPeekAtLastError();
+    if (e == cudaSuccess) e = cudaPeekAtLastError();
     if (e != cudaSuccess) return noalloc_fail(CMAG_ERR_CUDA, "sort launch (or an earlier pending error)", e);
     // wait for the sort and read its device-side check word
     uint32_t bits = 0;

@@ -1940,8 +1940,12 @@ int cmag_sort_particles(uint32_t *d_hash, uint32_t *d_index, uint32_t n, uint32_
     uint32_t *err = nullptr;
     CM_CUDA(nullptr, cudaHostGetDevicePointer((void **)&err, c.err, 0));
     CM_CUDA(nullptr, cudaMemsetAsync(c.ws, 0, sort_head_words() * sizeof(uint32_t), st));
-    launch_sort(d_hash, d_index, c.keys, c.vals, n, passes, sort_workspace_view(c.ws, n), err, st);
-    CM_CUDA(nullptr, cudaStreamSynchronize(st));
+    const cudaError_t launched =
+        launch_sort(d_hash, d_index, c.keys, c.vals, n, passes, sort_workspace_view(c.ws, n), err, st);
+    // (the workspace is idle again before the next call, also where a launch failed)
+    const cudaError_t waited = cudaStreamSynchronize(st);
+    CM_CUDA(nullptr, launched);
+    CM_CUDA(nullptr, waited);
     const uint32_t bits = *(volatile uint32_t *)c.err;
     if (bits)
         return fail(nullptr, CMAG_ERR_DEVICE,
