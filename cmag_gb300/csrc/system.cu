@@ -1001,11 +1001,18 @@ int cmag_system_create(const cmag_sph_params *params, uint32_t n, cmag_system **
         for (int a = 0; a < 3; ++a) s->wc_nb[a] = (params->grid_size[a] + 3u) / 4u;
         const size_t marks = sizeof(uint32_t) * (size_t)s->wc_nb[0] * s->wc_nb[1] * s->wc_nb[2];
         void **bufs[4] = {(void **)&s->wc_entry, (void **)&s->wc_snap, (void **)&s->wc_mark, (void **)&s->wc_state};
-        const size_t sizes[4] = {f4, 2 * f4, marks, 4 * sizeof(uint32_t)};  // snapshots, then nval
-        bool ok = true;
-        for (int k = 0; k < 4 && ok; ++k)
-            ok = cudaMalloc(bufs[k], sizes[k]) == cudaSuccess && cudaMemset(*bufs[k], 0, sizes[k]) == cudaSuccess;
-        if (!ok) {
+        // behind the snapshots the scratch of the interpolation and feature walks, where
+        // there is room for both (else it is made on first use)
+        bool ok = false;
+        for (size_t scratch : {f4, (size_t)0}) {
+            const size_t sizes[4] = {f4, f4 + scratch, marks, 4 * sizeof(uint32_t)};
+            ok = true;
+            for (int k = 0; k < 4 && ok; ++k)
+                ok = cudaMalloc(bufs[k], sizes[k]) == cudaSuccess && cudaMemset(*bufs[k], 0, sizes[k]) == cudaSuccess;
+            if (ok) {
+                if (scratch) s->nval = s->wc_snap + n;
+                break;
+            }
             (void)cudaGetLastError();
             for (int k = 0; k < 4; ++k) {
                 if (*bufs[k]) cudaFree(*bufs[k]);
@@ -1013,7 +1020,6 @@ int cmag_system_create(const cmag_sph_params *params, uint32_t n, cmag_system **
             }
         }
         s->wc_on = ok;
-        if (ok) s->nval = s->wc_snap + n;
     }
     if (rc != CMAG_OK) {
         std::string msg = s->last_error;

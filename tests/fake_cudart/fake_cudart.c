@@ -1,6 +1,7 @@
-/* The CUDA runtime calls that the library's sort makes, answered on the host and preloaded
- * before the real runtime: device memory is host memory, kernels do not run, and a call
- * chosen by the test (fake_fail) returns an error in place of the real one. */
+/* The CUDA runtime calls that the library's sort and the creation of a system make, answered
+ * on the host and preloaded before the real runtime: device memory is host memory, kernels
+ * do not run, and a call chosen by the test (fake_fail, fake_memory) returns an error in
+ * place of the real one. */
 #include <stdlib.h>
 #include <string.h>
 
@@ -64,10 +65,44 @@ int cudaDeviceGetAttribute(int *value, int attribute, int device)
     *value = 152;
     return kOk;
 }
-int cudaMalloc(void **p, size_t bytes) { return (*p = malloc(bytes)) ? kOk : 2; }
+/* device memory in use, and how much there is (-1: as much as asked for) */
+static long long g_used = 0, g_limit = -1;
+void fake_memory(long long limit) { g_limit = limit; }
+long long fake_used(void) { return g_used; }
+int cudaMalloc(void **p, size_t bytes)
+{
+    long long *block;
+    *p = NULL;
+    if (g_limit >= 0 && g_used + (long long)bytes > g_limit) return raise_error(2);
+    if (!(block = malloc(bytes + 64))) return raise_error(2);
+    block[0] = (long long)bytes;
+    g_used += (long long)bytes;
+    *p = (char *)block + 64;
+    return kOk;
+}
 int cudaFree(void *p)
 {
-    free(p);
+    if (p) {
+        long long *block = (long long *)((char *)p - 64);
+        g_used -= block[0];
+        free(block);
+    }
+    return kOk;
+}
+int cudaMemset(void *p, int value, size_t bytes)
+{
+    memset(p, value, bytes);
+    return kOk;
+}
+int cudaStreamCreateWithFlags(void **stream, unsigned flags)
+{
+    (void)flags;
+    *stream = &g_used;
+    return kOk;
+}
+int cudaStreamDestroy(void *stream)
+{
+    (void)stream;
     return kOk;
 }
 int cudaHostAlloc(void **p, size_t bytes, unsigned flags)
