@@ -63,6 +63,12 @@ struct cmag_system {
     int last_stage = CMAG_STAGE_INTEGRATE;
 
     int g_density = 1, g_force = 1;  // lanes per particle (cmag_system_autotune)
+    // what the autotuner found for the staged step of a scene that it left to the three
+    // launches (lanes 0: nothing); in_use: such steps run now (settle_lanes)
+    struct {
+        int g_density = 0, g_force = 0;
+        bool lists = false, in_use = false;
+    } tuned;
     uint32_t *nl_entry = nullptr, *nl_count = nullptr;  // interaction lists (when enabled)
     uint32_t nl_cap = 0;
     // lists kept over several steps (cmag_system_set_verlet): skin in particle
@@ -742,9 +748,27 @@ bool small_form(cmag_system *s)  // whatever the lanes
 }
 bool small_steps(cmag_system *s) { return s->g_density == 1 && s->g_force == 1 && small_form(s); }
 
+// An autotuned small scene takes one lane while its steps are three launches, and the
+// lanes and lists found for the staged step while something (a closure, stage timing,
+// graphs off) asks for that.
+void settle_lanes(cmag_system *s)
+{
+    auto &t = s->tuned;
+    if (t.g_density == 0 || s->vl_skin > 0.0f) return;
+    const bool staged = !small_form(s);
+    if (staged == t.in_use) return;
+    t.in_use = staged;
+    s->g_density = staged ? t.g_density : 1;
+    s->g_force = staged ? t.g_force : 1;
+    if (!staged) free_lists(s);
+    else if (t.lists && alloc_lists(s) != CMAG_OK) s->last_error.clear();  // (steps without lists)
+    invalidate_graph(s);
+}
+
 int do_step(cmag_system *s)
 {
     std::lock_guard<std::mutex> lock(s->launch_mu);
+    settle_lanes(s);
     bool small = small_steps(s);
     if (small) {  // on a stream that its owner captures a step is refused, as the staged one's graph is
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -1569,6 +1593,7 @@ int cmag_system_set_groups(cmag_system *s, int32_t gd, int32_t gf)
     if (!ok(gd) || !ok(gf)) return fail(s, CMAG_ERR_INVALID, "lanes per particle must be 1, 2 or 4");
     s->g_density = gd;
     s->g_force = gf;
+    s->tuned = {};
     invalidate_graph(s);
     return CMAG_OK;
 }
@@ -1649,8 +1674,13 @@ int cmag_system_autotune(cmag_system *s, int32_t reps)
         (void)cudaGetLastError();
     }
     // the trials time staged kernels; up to kSmallTuned particles a step of three
-    // launches, which takes one lane, beats the best of them
+    // launches, which takes one lane, beats the best of them, whose choice is kept for
+    // when steps are staged
+    s->tuned = {};
     if (s->n <= kSmallTuned && small_form(s)) {
+        s->tuned.g_density = gd;
+        s->tuned.g_force = gf;
+        s->tuned.lists = lists;
         gd = gf = 1;
         if (lists) free_lists(s);
         lists = false;
@@ -1671,6 +1701,7 @@ int cmag_system_set_neighbor_lists(cmag_system *s, int32_t enable)
     if (!s) return fail(nullptr, CMAG_ERR_INVALID, "null handle");
     if (enable < 0) return fail(s, CMAG_ERR_INVALID, "enable must be 0, 1 or an entry count");
     s->vl_skin = 0.0f;  // per-step lists (or none): lists are no longer kept
+    s->tuned = {};
     int rc = enable ? alloc_lists(s, enable > 1 ? (uint32_t)enable : 0u) : free_lists(s);
     invalidate_graph(s);
     return rc;

@@ -359,7 +359,8 @@ int cmag_system_get_verlet(cmag_system *s, float *skin, uint32_t *rebuilds);
 /* Autotune: on the current state, time the density and force kernels for every
  * lane count and with interaction lists (`reps` launches each) and keep the
  * fastest (planar scenes of up to 10,000 particles keep one lane, whose step of three
- * launches is faster).  Both kernels are recomputed from scratch every step; the choice
+ * launches is faster; what was found for their staged step is taken by the first step
+ * after a closure, stage timing or graphs off ask for that).  Both kernels are recomputed from scratch every step; the choice
  * changes only the summation order of the lanes' partial sums. */
 int cmag_system_autotune(cmag_system *s, int32_t reps);
 
