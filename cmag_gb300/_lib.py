@@ -88,6 +88,7 @@ SIGNATURES = {
                                     ctypes.c_int),
     "cmag_sort_particles_noalloc_error": ([], ctypes.c_char_p),
     "cmag_testing_set_sort_spin_limit": ([ctypes.c_int32], ctypes.c_int),
+    "cmag_testing_small_step_blocks": ([c_sys, c_u32p], ctypes.c_int),
     "cmag_system_colors": ([c_sys, c_f32p], ctypes.c_int),
     "cmag_system_render_ppm": ([c_sys, ctypes.c_char_p, c_u32, c_u32], ctypes.c_int),
     # batches

@@ -1696,6 +1696,15 @@ int cmag_system_autotune(cmag_system *s, int32_t reps)
     return CMAG_OK;
 }
 
+int cmag_testing_small_step_blocks(cmag_system *s, uint32_t *blocks)
+{
+    if (!s || !blocks) return fail(s, CMAG_ERR_INVALID, "null argument");
+    std::lock_guard<std::mutex> lock(s->launch_mu);
+    settle_lanes(s);
+    *blocks = small_steps(s) ? s->small_cluster : 0u;
+    return CMAG_OK;
+}
+
 int cmag_system_set_neighbor_lists(cmag_system *s, int32_t enable)
 {
     if (!s) return fail(nullptr, CMAG_ERR_INVALID, "null handle");

@@ -413,6 +413,9 @@ const char *cmag_sort_particles_noalloc_error(void);
  * give up at once, so tests can reach the failure path without a real stall: the
  * sort then returns CMAG_ERR_DEVICE and its output is wrong but stays in bounds. */
 int cmag_testing_set_sort_spin_limit(int32_t polls);
+/* For tests: blocks of the sorting cluster of the next step where that is a step of three
+ * launches, 0 where it is staged. */
+int cmag_testing_small_step_blocks(cmag_system *s, uint32_t *blocks);
 
 /* ---- headless colours and point view ----------------------------------- */
 /* The Demo programs' colour buffers without OpenGL: per particle (original
