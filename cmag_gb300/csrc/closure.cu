@@ -290,19 +290,19 @@ __device__ __forceinline__ uint32_t lds32(const __nv_bfloat16 *p)
 }
 
 // one hidden layer: c[nt] = bias + A x W^T over KT k-tiles; W rows of `stride` BF16
-template <int KT, int NT>
+template <int KT>
 __device__ __forceinline__ void hidden_layer(const __nv_bfloat16 *W, int stride, const float *b,
-                                             const uint32_t (&a)[KT][4], float (&c)[NT][4], int g, int t)
+                                             const uint32_t (&a)[KT][4], float (&c)[8][4], int g, int t)
 {
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
+    for (int nt = 0; nt < 8; ++nt) {
         c[nt][0] = c[nt][2] = b[nt * 8 + 2 * t];
         c[nt][1] = c[nt][3] = b[nt * 8 + 2 * t + 1];
     }
 #pragma unroll
     for (int kt = 0; kt < KT; ++kt)
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
+        for (int nt = 0; nt < 8; ++nt) {
             const __nv_bfloat16 *row = W + (nt * 8 + g) * stride + kt * 16 + 2 * t;
             mma16816(c[nt], a[kt], lds32(row), lds32(row + 8));
         }
@@ -518,11 +518,10 @@ __device__ __forceinline__ void store_parts(__nv_bfloat16 *at, int plane, float 
 
 // c = activations of a layer (pre-activations in c): BF16 activations of the warp's 16
 // rows to h (its row 0 and first column), slopes to c.
-template <int NT>
-__device__ __forceinline__ void activate(float (&c)[NT][4], __nv_bfloat16 *h, int g, int t)
+__device__ __forceinline__ void activate(float (&c)[4][4], __nv_bfloat16 *h, int g, int t)
 {
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
+    for (int nt = 0; nt < 4; ++nt) {
         float a[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -610,8 +609,8 @@ __device__ __forceinline__ void mma_add(float (&c)[4], const uint32_t (&a)[4], u
 
 // c = d W for the warp's 16 rows (W: its first column): the deltas of the layer below
 // before its slopes; the small parts first.
-template <bool MAIN, int NT>
-__device__ __forceinline__ void backward_part(const __nv_bfloat16 *W, const __nv_bfloat16 *d, float (&c)[NT][4],
+template <bool MAIN>
+__device__ __forceinline__ void backward_part(const __nv_bfloat16 *W, const __nv_bfloat16 *d, float (&c)[4][4],
                                               int lane)
 {
     const int r = lane & 7, q = lane >> 3;
@@ -620,7 +619,7 @@ __device__ __forceinline__ void backward_part(const __nv_bfloat16 *W, const __nv
         uint32_t a[4];
         load_matrices(a, d + (r + (q & 1) * 8) * kHStride + kt * 16 + (q >> 1) * 8);
 #pragma unroll
-        for (int nt = 0; nt < NT; nt += 2) {
+        for (int nt = 0; nt < 4; nt += 2) {
             uint32_t w[4];
             load_matrices_trans(w, W + (kt * 16 + (q & 1) * 8 + r) * kWStride + nt * 8 + (q >> 1) * 8);
             mma_add<MAIN>(c[nt], a, w[0], w[1]);
@@ -628,12 +627,11 @@ __device__ __forceinline__ void backward_part(const __nv_bfloat16 *W, const __nv
         }
     }
 }
-template <int NT>
-__device__ __forceinline__ void backward_layer(const __nv_bfloat16 *W, const __nv_bfloat16 *d, float (&c)[NT][4],
+__device__ __forceinline__ void backward_layer(const __nv_bfloat16 *W, const __nv_bfloat16 *d, float (&c)[4][4],
                                                int lane)
 {
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.0f;
+    for (int nt = 0; nt < 4; ++nt) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.0f;
 #pragma unroll 1
     for (int part = 2; part >= 1; --part) backward_part<false>(W, d + part * kPlane, c, lane);
     backward_part<true>(W, d, c, lane);

@@ -1,5 +1,6 @@
 // pair_terms.cuh -- the force of one candidate pair, without branches on its distance,
-// for the three-launch step of small scenes (small_step.cu).
+// for the three-launch step of small planar scenes (small_step.cu).  Every particle of such
+// a scene has the same z and no z velocity, so each z term is an exact zero and is left out.
 //
 // The same operations as the scalar pair of the force pass (force.cu), so that terms
 // added in the same order give the same bits.  The force pass keeps its own form,
@@ -24,8 +25,8 @@ struct PairSelf {
 // DamBreak: sum += a r.  Poiseuille: sum += a r, then b v.  Peristalsis: pressure
 // sum += a r, viscous sum += b v.
 struct PairTerms {
-    float a, rx, ry, rz;
-    float b, vx, vy, vz;
+    float a, rx, ry;
+    float b, vx, vy;
 };
 
 // Lennard-Jones wall force over r (fluid_kernel.cu:199-207).
@@ -38,8 +39,8 @@ __device__ __forceinline__ float wall_factor(const DevParams &p, float d2)
 }
 
 // The terms of an interacting fluid pair (Poiseuille, Peristalsis: any pair) at
-// distance (t.rx, t.ry, t.rz), squared d2, from candidate values pj, vj, aj.
-template <int SYS, bool PLANAR>
+// distance (t.rx, t.ry), squared d2, from candidate values pj, vj, aj.
+template <int SYS>
 __device__ __forceinline__ void pair_factors(const DevParams &p, const PairSelf &s, const float4 &pj, float d2,
                                              const float4 &vj, const float2 &aj, PairTerms &t)
 {
@@ -48,8 +49,7 @@ __device__ __forceinline__ void pair_factors(const DevParams &p, const PairSelf 
     if (SYS == CMAG_DAMBREAK) {
         // pressure + Monaghan viscosity (fluid_kernel.cu:221-237)
         float q = s.aux.x + aj.x;
-        const float vxy = __fmaf_rn(s.vel.y - vj.y, t.ry, (s.vel.x - vj.x) * t.rx);
-        const float vij = PLANAR ? vxy : __fmaf_rn(s.vel.z - vj.z, t.rz, vxy);
+        const float vij = __fmaf_rn(s.vel.y - vj.y, t.ry, (s.vel.x - vj.x) * t.rx);
         if (vij < 0.0f) {
             // viscosity 2 alpha h c0 v_ij / ((rho_i + rho_j)(r^2 + eps^2))
             q -= __fdividef(p.av_coeff * vij, (s.aux.y + aj.y) * (d2 + p.av_eps2));
@@ -59,7 +59,6 @@ __device__ __forceinline__ void pair_factors(const DevParams &p, const PairSelf 
     }
     t.vx = s.vel.x - vj.x;
     t.vy = s.vel.y - vj.y;
-    t.vz = s.vel.z - vj.z;
     if (SYS == CMAG_POISEUILLE && pj.w == 1.0f && (pj.y > p.wall_top || pj.y < p.wall_bottom)) {
         // Morris viscosity with wall extrapolation (poiseuilleFlowKernel.cu:184-208)
         const bool top = pj.y > p.wall_top;
@@ -68,7 +67,6 @@ __device__ __forceinline__ void pair_factors(const DevParams &p, const PairSelf 
         const float beta = fminf(1000.0f, 1.0f + __fdividef(db, da));
         t.vx = beta * s.vel.x;
         t.vy = beta * s.vel.y;
-        t.vz = beta * s.vel.z;
     }
     // pressure (poiseuilleFlowKernel.cu:236-245, PeristalsisPressureForce.cu:39-43)
     // and viscous (PeristalsisViscousForce.cu:206-213) factors
@@ -76,37 +74,31 @@ __device__ __forceinline__ void pair_factors(const DevParams &p, const PairSelf 
     t.b = s.visc_i * aj.y * g;
 }
 
-// Squared distance of the particle from candidate pj seen through image shift
-// (sx, sy, sz); the relative position in t.
-template <int SYS, bool PLANAR>
-__device__ __forceinline__ float pair_distance(const PairSelf &s, const float4 &pj, float sx, float sy, float sz,
-                                               PairTerms &t)
+// Squared distance of the particle from candidate pj seen through image shift (sx, sy);
+// the relative position in t.
+template <int SYS>
+__device__ __forceinline__ float pair_distance(const PairSelf &s, const float4 &pj, float sx, float sy, PairTerms &t)
 {
-    const float3 rv = walk::rel<SYS>(s.pos, pj, sx, sy, sz);
-    // planar scenes: every particle has the same z and no z velocity, so each z
-    // term is an exact zero and is left out (same bits)
+    const float3 rv = walk::rel<SYS>(s.pos, pj, sx, sy, 0.0f);
     t.rx = rv.x;
     t.ry = rv.y;
-    t.rz = PLANAR ? 0.0f : rv.z;
-    return PLANAR ? __fmaf_rn(t.ry, t.ry, t.rx * t.rx)
-                  : __fmaf_rn(t.rz, t.rz, __fmaf_rn(t.ry, t.ry, t.rx * t.rx));
+    return __fmaf_rn(t.ry, t.ry, t.rx * t.rx);
 }
 
 // The terms of candidate j with its position, velocity and aux data at hand (loaded
 // together, so that several candidates' loads are in flight); zeros and false when
 // the pair contributes nothing.
-template <int SYS, bool PLANAR, bool TRIM>
+template <int SYS, bool TRIM>
 __device__ __forceinline__ bool pair_terms(const DevParams &p, const PairSelf &s, uint32_t j, const float4 &pj,
-                                              const float4 &vj, const float2 &aj, float sx, float sy, float sz,
-                                              PairTerms &t)
+                                           const float4 &vj, const float2 &aj, float sx, float sy, PairTerms &t)
 {
-    const float d2 = pair_distance<SYS, PLANAR>(s, pj, sx, sy, sz, t);
+    const float d2 = pair_distance<SYS>(s, pj, sx, sy, t);
     // (a coincident pair has no direction: it contributes nothing)
     const bool wall = SYS == CMAG_DAMBREAK && pj.w != (float)CMAG_FLUID;
     // a wall without cut-off at a distance that is not a number: the walk takes it, lists
     // do not hold it
     const bool hit = j != s.i && d2 != 0.0f && (d2 < p.support2 || (wall && !TRIM && (!s.lists || d2 > 0.0f)));
-    pair_factors<SYS, PLANAR>(p, s, pj, d2, vj, aj, t);
+    pair_factors<SYS>(p, s, pj, d2, vj, aj, t);
     if (wall) t.a = wall_factor(p, d2);
     if (!hit) t = PairTerms{};
     return hit;

@@ -1,6 +1,6 @@
 // particle_motion.cuh -- time integration of one particle and the Peristalsis
 // phase machine, shared by the integration kernels (integrate.cu) and the
-// one-launch step of small scenes (small_step.cu).
+// three-launch step of small scenes (small_step.cu).
 //
 //   integrate                    DamBreak.Core/fluid_kernel.cu:323-366
 //   integratePoiseuilleSystemD   Poiseuille.Core/poiseuilleFlowKernel.cu:311-348

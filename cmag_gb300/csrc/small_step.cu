@@ -534,8 +534,8 @@ __device__ __forceinline__ bool add_row_forces(const DevParams &p, const SmallSt
 #pragma unroll
         for (uint32_t u = 0; u < U; ++u) {
             PairTerms t;
-            const bool hit = pair_terms<SYS, true, TRIM>(p, self, j[u], q[u], v[u], x[u],
-                                                            k0 + u < row.n0 ? row.sx0 : row.sx1, row.sy, 0.0f, t);
+            const bool hit = pair_terms<SYS, TRIM>(p, self, j[u], q[u], v[u], x[u],
+                                                   k0 + u < row.n0 ? row.sx0 : row.sx1, row.sy, t);
             Slot<SYS>::put(s + gr.slot(min(at, (uint32_t)Slot<SYS>::count), gr.lane, Slot<SYS>::words), t);
             at += hit ? 1u : 0u;
         }
@@ -562,10 +562,10 @@ __device__ __noinline__ float add_long_row_forces(const DevParams &p, const Smal
                 const uint32_t j = base + gr.lane < e ? base + gr.lane : self.i;
                 PairTerms t{};
                 const float4 q = __ldg(a.spos + j);
-                const float d2 = pair_distance<SYS, true>(self, q, sx, row.sy, 0.0f, t);
+                const float d2 = pair_distance<SYS>(self, q, sx, row.sy, t);
                 const bool out = !(d2 < p.support2) && (SYS != CMAG_DAMBREAK || TRIM || q.w == (float)CMAG_FLUID);
                 if (gr.all(out || j == self.i)) continue;  // out of reach: nothing to add
-                pair_terms<SYS, true, TRIM>(p, self, j, q, __ldg(a.svel + j), __ldg(a.aux + j), sx, row.sy, 0.0f, t);
+                pair_terms<SYS, TRIM>(p, self, j, q, __ldg(a.svel + j), __ldg(a.aux + j), sx, row.sy, t);
                 Slot<SYS>::put(s + gr.slot(0, gr.lane, Slot<SYS>::words), t);
                 gr.sync();
                 if (gr.lane < Slot<SYS>::lanes)
