@@ -867,10 +867,9 @@ __device__ __forceinline__ void update_image(uint32_t *image, int k, float v)
 // The gradient of parameter k: the sum of its copies.
 __device__ __forceinline__ float gradient_of(const float *grad, int k)
 {
-    double g = 0.0;
-#pragma unroll
-    for (int c = 0; c < kGradCopies; ++c) g += (double)grad[c * kGradStride + k];
-    return (float)g;
+    static_assert(kGradCopies == 4, "added in pairs");
+    grad += k;
+    return (grad[0] + grad[kGradStride]) + (grad[2 * kGradStride] + grad[3 * kGradStride]);
 }
 
 // Leaves the gradient in its first copy.

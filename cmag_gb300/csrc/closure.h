@@ -63,8 +63,8 @@ void launch_interpolate(const DevParams &p, const float4 *spos, const float2 *au
 void launch_closure_forward(const ClosureView &c, const float *feat, uint32_t n,
                             __nv_bfloat16 *xb, float *out, cudaStream_t st);
 // The blocks of a backward pass add their gradients to kGradCopies FP32 copies in turn,
-// so that a chain of rounded additions is a quarter as long; the copies are summed in
-// 64 bits where the gradient is used.  kGradStride floats apart (8-byte aligned).
+// so that a chain of rounded additions is a quarter as long; the copies are summed where
+// the gradient is used.  kGradStride floats apart (8-byte aligned).
 constexpr int kGradCopies = 4;
 constexpr int kGradStride = (kClosureParams + 1) & ~1;
 // Loss 0.5/n sum |y - t|^2 over n rows (t: targets, n x 3) added to *loss and its
