@@ -591,7 +591,7 @@ __device__ __forceinline__ void mma16816_zero(float (&d)[4], const uint32_t (&a)
 
 // c += A B, MAIN: for the main part of a delta.  The tensor cores truncate a running sum
 // at every addition, always towards zero; over a chain of products that shrinks the sum
-// by up to 1e-7 of it.  So the main part's products are summed from zero, 16 at a time
+// by about 1e-7 of it.  So the main part's products are summed from zero, 16 at a time
 // (their 16 bits each mostly fit), and added here in FP32, rounded to nearest.  The small
 // parts (2^-8 and 2^-16 of the main one) lose nothing that counts in a chain.
 template <bool MAIN>

@@ -177,14 +177,18 @@ void launch_verlet_check(const float4 *pos, const float4 *xb, uint32_t start, ui
 
 // ---- the step of a small planar scene in three launches (small_step.cu) ----------
 // Largest scene that takes it.  The neighbour loops' lanes cost several times the
-// instructions of one lane, which pays while the GPU has idle issue slots: three
-// solvers in turn, us per step of each, here / staged: 352 particles 6.2 / 15.7,
-// 3,840 11 / 21, 16,384 18.6 / 23.8; with 8 lanes 21,200 22.3 / 19.8, 34,800 33 / 21.
+// instructions of one lane, which pays while the GPU has idle issue slots.  The line lies
+// where three solvers in turn stop gaining (us per step of each, here / staged, four lanes
+// from 12,000 on: 352 particles 6.3 / 14.9, 3,840 10.4 / 20.3, 8,702 15.2 / 22.8, 16,384
+// 19.1 / 24.1, 16,918 24.0 / 24.4, 16,960 17.9 / 19.0, 19,840 20.4 / 19.1, 19,990
+// 26.9 / 25.8, 20,480 23.8 / 24.5, 29,200 27.2 / 20.7, 34,838 39.2 / 27.5); one solver
+// alone would still gain a little beyond it (19,990 50 / 63, 20,480 49 / 60, 29,200
+// 48.7 / 49.2, 34,838 75 / 65).
 constexpr uint32_t kSmallParticles = 18000;
 // Up to here the three launches also beat the staged step at the lanes the autotuner
-// finds (us a step of one solver, three launches / tuned stages: Poiseuille 4480
-// particles 20.0 / 28.7, dam break 8702 31.3 / 43.7, 16,918 44.8 / 37.9, Peristalsis
-// 16,384 41.0 / 35.9).
+// finds (us a step of one solver, three launches / tuned stages: 352 particles 17.4 / 22.6,
+// Poiseuille 4480 20 / 28, dam break 8702 31.3 / 39.3, Poiseuille 10,800 30.2 / 28.7, dam
+// break 12,158 43 / 37, 16,918 48.5 / 44.1, Peristalsis 16,384 40.5 / 35.3).
 constexpr uint32_t kSmallTuned = 10000;
 constexpr uint32_t kSmallCells = 1u << 18;  // the sort's cluster scans them in a few us
 // The arrays of launch_hash .. launch_integrate; rank may alias idx.

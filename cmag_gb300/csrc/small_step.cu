@@ -10,20 +10,20 @@
 //     for the block's writes) instead of launches, the scan's block totals through
 //     distributed shared memory.  Bound by the latency of its five stages (10-17 us).
 //     512 threads a block: at 1024 the cluster waits for 16 SMs that are nearly empty
-//     when other solvers run beside it (20.5 against 25 us a step, 16,384 particles);
+//     when other solvers run beside it (16,384 particles, 8 lanes: 20.5 against 25 us a step);
 //   * the density and the force give each particle 8 lanes (4 in the larger scenes),
 //     one per row of its cell box, so a particle's cell lookups and loads are in
 //     flight together.  Bound by that latency up to about 10,000 particles, then by
 //     instruction issue;
 //   * the force launch integrates its particles too.
-// One solver alone, us per step: Poiseuille 4,480 particles 41 -> 20.5, dam break
-// 8,702 61 -> 32, Peristalsis 16,384 58.5 -> 43; three solvers in turn, where the
-// host's 15 us a step counts: 16.5 -> 8.5, 37.8 -> 31.7, 23.8 -> 18.6.
+// One solver alone, us per step, staged -> here: Poiseuille 4,480 particles 43 -> 20, dam
+// break 8,702 61 -> 31, Peristalsis 16,384 60 -> 41; three solvers in turn, where the
+// host's 15 us a step counts: 15.6 -> 8.5, 22.8 -> 15.2, 24.1 -> 19.1.
 //
 // Same bits as the staged step with one lane per particle: the lanes leave their
 // candidates' terms in shared memory, and one lane per sum adds them in the order of
-// the one-lane walk.  (The staged step's lanes add partial sums of their rows, which
-// rounds differently.)
+// the one-lane walk, NaN of particles at no finite place included.  (The staged step's
+// lanes add partial sums of their rows, which rounds differently.)
 #include <cuda_runtime.h>
 
 #include "kernels.h"
@@ -172,9 +172,11 @@ __global__ void __launch_bounds__(kSortBlock, 1) k_small_sort(DevParams p, Small
 
 // 8 lanes take a box of 7 rows at once: the shortest chain, and the form of scenes up to
 // kWideParticles.  4 lanes take it in two batches with half the warps: above that line,
-// where solvers that share the GPU compete for issue slots (us per step of each of three
-// solvers, 8 lanes / 4: 4480 particles 8.5 / 10.4, 8702 15.0 / 16.3, 16,384 20.5 / 18.6,
-// 16,960 21.0 / 17.9; one solver alone 19.6 / 29.2, 31.3 / 38.4, 41.0 / 43.6, 34.8 / 33.1).
+// where solvers that share the GPU compete for issue slots (us per step, 8 lanes / 4, three
+// solvers in turn; one alone: Poiseuille 4480 particles 8.5 / 10.0; 19.3 / 29.2, dam break
+// 8702 15.2 / 16.3; 31.5 / 38.8, Poiseuille 10,800 14.5 / 12.8; 30.2 / 31.2, dam break 12,158
+// 19.0 / 19.3; 40.7 / 42.6, Peristalsis 16,384 21.0 / 19.1; 39.4 / 40.6, Poiseuille 16,960
+// 21.0 / 17.9; 34.8 / 33.4).
 constexpr uint32_t kWideParticles = 12000;
 constexpr int kSlots = 8;            // terms of a row held at once
 constexpr uint32_t kRowMost = 32;    // candidates of a row that one lane takes

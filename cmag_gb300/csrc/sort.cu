@@ -192,8 +192,8 @@ __device__ __forceinline__ uint32_t sum_back(const volatile uint32_t *st, uint32
 //     inclusive prefix): two or three round trips, where looking back tile by tile took
 //     ten to twelve.
 //   * The pairs are put in digit order in shared memory and written as runs.
-// 954,860 pairs of 23 bits: 25.7 -> 18.5 us a pass (ncu), the whole call 144 -> 97 us;
-// 4 million of 30 bits 392 -> 288 us, 2,000 of 12 bits 62 -> 56 us.
+// 954,860 pairs of 23 bits: 25.7 -> 17-20 us a pass (ncu), the whole call 144-153 ->
+// 97-105 us (boxes differ); 4 million of 30 bits 392 -> 288 us, 2,000 of 12 bits 62 -> 56 us.
 template <int kItems>
 __global__ void __launch_bounds__(kSortThreads, 1)
     k_onesweep(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
